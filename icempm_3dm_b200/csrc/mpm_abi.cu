@@ -114,6 +114,9 @@ struct mpm_handle {
     int adj_force_cap = 0;
     std::vector<double*> adj_gcache;  // P2G grid of each substep of the segment being reversed
     double* adj_rmv = nullptr;        // return-map VJP of the crushed points (10 x pitch)
+    int* adj_rml = nullptr;           // crushed points of each substep of the segment (pitch per substep)
+    int* adj_rmc = nullptr;           // and their counts
+    int adj_rm_cap = 0;               // substeps the two hold
 
 
     // animation-frame records (mpm_frame_records), allocated on first use
@@ -256,7 +259,7 @@ void free_all(mpm_handle* h) {
     cudaFree(h->adj_force);
     for (double* c : h->adj_gcache) cudaFree(c);
     h->adj_gcache.clear();
-    cudaFree(h->adj_rmv);
+    cudaFree(h->adj_rmv); cudaFree(h->adj_rml); cudaFree(h->adj_rmc);
     for (int* p : h->scan_levels) cudaFree(p);
     h->scan_levels.clear();
     cudaFree(h->fr_f); cudaFree(h->fr_status); cudaFree(h->fr_last); cudaFree(h->fr_i); cudaFree(h->fr_rec);
@@ -385,7 +388,9 @@ int launch_g2p2g_mixed(mpm_handle* h, int do_p2g, int record_pq, int store_vc) {
     return MPM_OK;
 }
 
-int launch_g2p(mpm_handle* h, int record_pq) {
+// list, count (FP64 modes, may be null): where the crushed points are listed
+// (count zeroed by the caller) instead of the handle's own list.
+int launch_g2p(mpm_handle* h, int record_pq, int* list = nullptr, int* count = nullptr) {
     const int n = (int)h->n;
     if (n == 0) return MPM_OK;
     if (is_mixed(h)) {
@@ -394,18 +399,20 @@ int launch_g2p(mpm_handle* h, int record_pq) {
     }
     const unsigned nb = blocks_for(n, 128);
     const int cur = h->rm_parity;
-    h->rm_parity ^= 1;
-    int* const cnt = h->rm_counts + cur;
-    int* const next = h->rm_counts + (cur ^ 1);
+    if (!list) h->rm_parity ^= 1;
+    int* const cnt = list ? count : h->rm_counts + cur;
+    // the counter the next launch on the handle's own list appends to is zero already
+    int* const next = h->rm_counts + (list ? cur : cur ^ 1);
+    if (!list) list = h->rm_list;
     const int rb = h->num_sms * 4;
     if (h->precision == MPM_PRECISION_FP64) {
         k_g2p_f64<SvdF32><<<nb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, n, h->grid, record_pq, h->err,
-                                                    h->rm_list, cnt);
-        k_return_map_f64<SvdF32><<<rb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, h->p0, h->rm_list, cnt, next);
+                                                    list, cnt);
+        k_return_map_f64<SvdF32><<<rb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, h->p0, list, cnt, next);
     } else {
         k_g2p_f64<SvdF64><<<nb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, n, h->grid, record_pq, h->err,
-                                                    h->rm_list, cnt);
-        k_return_map_f64<SvdF64><<<rb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, h->p0, h->rm_list, cnt, next);
+                                                    list, cnt);
+        k_return_map_f64<SvdF64><<<rb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, h->p0, list, cnt, next);
     }
     CK_LAUNCH(h, "g2p kernel");
     return MPM_OK;
@@ -2076,8 +2083,10 @@ namespace {
 size_t state_bytes(const mpm_handle* h) { return sizeof(double) * MPM_N_PTS_ARRAYS * h->pitch; }
 
 // One FP64 substep of Model3D::Step on the particle rows at h->pts;
-// p2g_copy (may be null) receives the grid after P2G (4 x gstride doubles).
-int fp64_substep(mpm_handle* h, double* force3, double* p2g_copy = nullptr) {
+// p2g_copy (may be null) receives the grid after P2G (4 x gstride doubles),
+// rm_list and rm_count (zeroed) the points that it crushed.
+int fp64_substep(mpm_handle* h, double* force3, double* p2g_copy = nullptr, int* rm_list = nullptr,
+                 int* rm_count = nullptr) {
     SimParams3D& p = h->prms;
     p.SimulationTime += p.InitialTimeStep;
     p.indenter_x = p.indenter_x_initial + p.SimulationTime * p.IndVelocity;
@@ -2089,7 +2098,7 @@ int fp64_substep(mpm_handle* h, double* force3, double* p2g_copy = nullptr) {
                               h->stream));
     if ((r = launch_update(h, p.indenter_x, p.indenter_y, force3))) return r;
     const int record = (p.SimulationStep % p.UpdateEveryNthStep) == 0;
-    if ((r = launch_g2p(h, record))) return r;
+    if ((r = launch_g2p(h, record, rm_list, rm_count))) return r;
     p.SimulationStep += 1;
     return MPM_OK;
 }
@@ -2112,6 +2121,16 @@ int ensure_adjoint_buffers(mpm_handle* h, int nsteps, int every) {
         h->adj_gcache.push_back(b);
     }
     h->ckpt_prms.resize(nck);
+    if (every > h->adj_rm_cap) {
+        CK(h, cudaStreamSynchronize(h->stream));
+        cudaFree(h->adj_rml);
+        cudaFree(h->adj_rmc);
+        h->adj_rml = h->adj_rmc = nullptr;
+        h->adj_rm_cap = 0;
+        CK(h, cudaMalloc(&h->adj_rml, sizeof(int) * h->pitch * (size_t)every));
+        CK(h, cudaMalloc(&h->adj_rmc, sizeof(int) * (size_t)every));
+        h->adj_rm_cap = every;
+    }
     if (!h->adj_A) {
         CK(h, cudaMalloc(&h->adj_A, sizeof(double) * ADJ_ROWS * h->pitch));
         CK(h, cudaMalloc(&h->adj_cgrad, sizeof(double) * h->pitch));
@@ -2247,11 +2266,13 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
         std::vector<SimParams3D> sp(s1 - s0);
         CK(h, cudaMemcpyAsync(h->seg[0], h->ckpt[j], state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
         h->prms = h->ckpt_prms[j];
+        CK(h, cudaMemsetAsync(h->adj_rmc, 0, sizeof(int) * (size_t)(s1 - s0), h->stream));
         for (int s = s0; s < s1 && !r; s++) {
             double* next = h->seg[s - s0 + 1];
             CK(h, cudaMemcpyAsync(next, h->seg[s - s0], state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
             h->pts = next;
-            r = fp64_substep(h, h->force_phase, h->adj_gcache[s - s0]);
+            r = fp64_substep(h, h->force_phase, h->adj_gcache[s - s0], h->adj_rml + h->pitch * (size_t)(s - s0),
+                             h->adj_rmc + (s - s0));
             sp[s - s0] = h->prms;   // holds this substep's indenter position
         }
         h->pts = pts_final;
@@ -2266,8 +2287,9 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
                                   h->stream));
             k_adj_update_record<256><<<blocks_for(dp.nodes, 256), 256, 0, h->stream>>>(dp, h->adj_g7, ix, iy);
             CK(h, cudaMemsetAsync(h->adj_gb7, 0, sizeof(double) * 7 * gs, h->stream));
-            k_adj_rm_vjp<128><<<blocks_for(n, 128), 128, 0, h->stream>>>(dp, q, Sn, Sn1, h->pitch, n, h->p0, h->adj_A,
-                                                                        h->adj_rmv, h->adj_cgrad, h->adj_Egrad);
+            k_adj_rm_vjp<128><<<h->num_sms * 4, 128, 0, h->stream>>>(
+                dp, q, Sn, Sn1, h->pitch, h->adj_rml + h->pitch * (size_t)(s - s0), h->adj_rmc + (s - s0), h->p0,
+                h->adj_A, h->adj_rmv, h->adj_cgrad, h->adj_Egrad);
             k_adj_g2p_rev<128><<<blocks_for(n, 128), 128, 0, h->stream>>>(dp, q, Sn, Sn1, h->pitch, n, h->adj_g7,
                                                                          h->adj_rmv, h->adj_A, h->adj_gb7);
             k_adj_node_rev<256><<<blocks_for(dp.nodes, 256), 256, 0, h->stream>>>(
