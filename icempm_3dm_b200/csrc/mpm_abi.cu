@@ -91,7 +91,7 @@ struct mpm_handle {
     void* mx = nullptr;
     float* p0f = nullptr;
     float4* gacc = nullptr;
-    unsigned long long* gacc_q = nullptr;   // the fixed-point accumulator when selected (4 per node)
+    unsigned long long* gacc_q = nullptr;   // the fixed-point accumulator when selected (4 arrays, dp.gstride apart)
     float4* gvel = nullptr;
     bool p2g_ready = false;           // gacc holds the P2G of the current state
     int num_sms = 148;
@@ -289,6 +289,8 @@ MixedState mixed_state(mpm_handle* h) {
     return m;
 }
 
+AccQ acc_q(const mpm_handle* h) { return AccQ{h->gacc_q, h->dp.gstride}; }
+
 // staging (FP64 SoA) -> mixed state; p0 (FP64) -> p0f
 int mixed_from_staging(mpm_handle* h) {
     if (!h->n) return MPM_OK;
@@ -318,7 +320,7 @@ int launch_p2g(mpm_handle* h) {
     if (n == 0) return MPM_OK;
     if (is_mixed(h)) {
         if (h->gacc_q)
-            k_p2g_mixed<<<blocks_for(n, 128), 128, 0, h->stream>>>(h->dp, mixed_state(h), n, AccQ{h->gacc_q}, h->err);
+            k_p2g_mixed<<<blocks_for(n, 128), 128, 0, h->stream>>>(h->dp, mixed_state(h), n, acc_q(h), h->err);
         else
             k_p2g_mixed<<<blocks_for(n, 128), 128, 0, h->stream>>>(h->dp, mixed_state(h), n, AccF4{h->gacc}, h->err);
         CK_LAUNCH(h, "p2g mixed");
@@ -334,7 +336,7 @@ int launch_update(mpm_handle* h, double ind_x, double ind_y, double* force3) {
     if (is_mixed(h)) {
         const unsigned nbm = blocks_for((long long)h->dp.node_hi - h->dp.node_lo, 256 * kUpdateNodesPerThread);
         if (h->gacc_q)
-            k_update_mixed<256><<<nbm, 256, 0, h->stream>>>(h->dp, AccQ{h->gacc_q}, h->gvel, ind_x, ind_y, h->sensor,
+            k_update_mixed<256><<<nbm, 256, 0, h->stream>>>(h->dp, acc_q(h), h->gvel, ind_x, ind_y, h->sensor,
                                                            force3);
         else
             k_update_mixed<256><<<nbm, 256, 0, h->stream>>>(h->dp, AccF4{h->gacc}, h->gvel, ind_x, ind_y, h->sensor,
@@ -357,7 +359,7 @@ int launch_return_map_mixed(mpm_handle* h, int do_p2g) {
     if (h->gacc_q)
         k_return_map_mixed<<<h->num_sms * 4, 128, 0, h->stream>>>(h->dp, mixed_state(h), h->rm_list,
                                                                   h->rm_counts + cur, h->rm_counts + (cur ^ 1),
-                                                                  AccQ{h->gacc_q}, do_p2g, h->err);
+                                                                  acc_q(h), do_p2g, h->err);
     else
         k_return_map_mixed<<<h->num_sms * 4, 128, 0, h->stream>>>(h->dp, mixed_state(h), h->rm_list,
                                                                   h->rm_counts + cur, h->rm_counts + (cur ^ 1),
@@ -378,7 +380,7 @@ int launch_g2p2g_mixed(mpm_handle* h, int do_p2g, int record_pq, int store_vc) {
     const size_t vsm = sizeof(float4) * (kFusedBlock / 32) * kVBoxNodes;
     if (h->gacc_q)
         k_g2p2g_mixed<<<blocks_for(n, kFusedBlock), kFusedBlock, vsm, h->stream>>>(
-            h->dp, mixed_state(h), n, h->gvel, AccQ{h->gacc_q}, do_p2g, record_pq, store_vc, h->err, h->rm_list,
+            h->dp, mixed_state(h), n, h->gvel, acc_q(h), do_p2g, record_pq, store_vc, h->err, h->rm_list,
             rm_count);
     else
         k_g2p2g_mixed<<<blocks_for(n, kFusedBlock), kFusedBlock, vsm, h->stream>>>(
@@ -421,7 +423,7 @@ int launch_g2p(mpm_handle* h, int record_pq, int* list = nullptr, int* count = n
 int reset_grid(mpm_handle* h) {
     if (is_mixed(h)) {
         if (h->gacc_q)
-            CK(h, cudaMemsetAsync(h->gacc_q, 0, sizeof(unsigned long long) * 4 * (size_t)h->dp.nodes, h->stream));
+            CK(h, cudaMemsetAsync(h->gacc_q, 0, sizeof(unsigned long long) * 4 * (size_t)h->dp.gstride, h->stream));
         else
             CK(h, cudaMemsetAsync(h->gacc, 0, sizeof(float4) * (size_t)h->dp.nodes, h->stream));
         h->p2g_ready = false;
@@ -781,8 +783,8 @@ int mpm_set_grid_accumulation(mpm_handle* h, int mode) {
     if (!is_mixed(h)) return mode == MPM_ACCUM_FLOAT ? MPM_OK : MPM_ERR_ARG;
     CK(h, cudaStreamSynchronize(h->stream));
     if (mode == MPM_ACCUM_FIXED && !h->gacc_q) {
-        CK(h, cudaMalloc(&h->gacc_q, sizeof(unsigned long long) * 4 * (size_t)h->dp.nodes));
-        CK(h, cudaMemsetAsync(h->gacc_q, 0, sizeof(unsigned long long) * 4 * (size_t)h->dp.nodes, h->stream));
+        CK(h, cudaMalloc(&h->gacc_q, sizeof(unsigned long long) * 4 * (size_t)h->dp.gstride));
+        CK(h, cudaMemsetAsync(h->gacc_q, 0, sizeof(unsigned long long) * 4 * (size_t)h->dp.gstride, h->stream));
     } else if (mode == MPM_ACCUM_FLOAT && h->gacc_q) {
         CK(h, cudaFree(h->gacc_q));
         h->gacc_q = nullptr;
@@ -1120,8 +1122,9 @@ int mpm_halo_pack(mpm_handle* h, int side, void* dst) {
     const long long off = halo_offset(h, side);
     if (is_mixed(h)) {
         if (h->gacc_q)
-            CK(h, cudaMemcpyAsync(dst, h->gacc_q + 4 * off, sizeof(unsigned long long) * 4 * hn,
-                                  cudaMemcpyDeviceToDevice, h->stream));
+            CK(h, cudaMemcpy2DAsync(dst, sizeof(unsigned long long) * hn, h->gacc_q + off,
+                                    sizeof(unsigned long long) * h->dp.gstride, sizeof(unsigned long long) * hn, 4,
+                                    cudaMemcpyDeviceToDevice, h->stream));
         else
             CK(h, cudaMemcpyAsync(dst, h->gacc + off, sizeof(float4) * hn, cudaMemcpyDeviceToDevice, h->stream));
         return MPM_OK;
@@ -1139,8 +1142,8 @@ int mpm_halo_add(mpm_handle* h, int side, const void* src) {
     if (!hn) return MPM_OK;
     const long long off = halo_offset(h, side);
     if (is_mixed(h) && h->gacc_q)
-        k_halo_add_q<<<blocks_for(4 * hn, 256), 256, 0, h->stream>>>(h->gacc_q, off, (int)hn,
-                                                                     static_cast<const unsigned long long*>(src));
+        k_halo_add_q<<<blocks_for(hn, 256), 256, 0, h->stream>>>(h->gacc_q, h->dp.gstride, off, (int)hn,
+                                                                 static_cast<const unsigned long long*>(src));
     else if (is_mixed(h))
         k_halo_add_f4<<<blocks_for(hn, 256), 256, 0, h->stream>>>(h->gacc, off, (int)hn,
                                                                   static_cast<const float4*>(src));
@@ -1920,11 +1923,11 @@ int mpm_testing_active_nodes(mpm_handle* h, long long* count) {
     const size_t nodes = (size_t)h->dp.nodes;
     long long c = 0;
     if (is_mixed(h) && h->gacc_q) {
-        std::vector<unsigned long long> g(4 * nodes);
-        CK(h, cudaMemcpyAsync(g.data(), h->gacc_q, sizeof(unsigned long long) * 4 * nodes, cudaMemcpyDeviceToHost,
+        std::vector<unsigned long long> g(nodes);
+        CK(h, cudaMemcpyAsync(g.data(), h->gacc_q, sizeof(unsigned long long) * nodes, cudaMemcpyDeviceToHost,
                               h->stream));
         CK(h, cudaStreamSynchronize(h->stream));
-        for (size_t i = 0; i < nodes; i++) c += g[4 * i] != 0ull;
+        for (size_t i = 0; i < nodes; i++) c += g[i] != 0ull;
     } else if (is_mixed(h)) {
         std::vector<float4> g(nodes);
         CK(h, cudaMemcpyAsync(g.data(), h->gacc, sizeof(float4) * nodes, cudaMemcpyDeviceToHost, h->stream));
@@ -1944,13 +1947,14 @@ int mpm_testing_download_grid(mpm_handle* h, double* out, int which) {
     if (!h || !out) return MPM_ERR_ARG;
     const size_t nodes = (size_t)h->dp.nodes;
     if (is_mixed(h) && h->gacc_q && !which) {
-        std::vector<unsigned long long> g(4 * nodes);
-        CK(h, cudaMemcpyAsync(g.data(), h->gacc_q, sizeof(unsigned long long) * 4 * nodes, cudaMemcpyDeviceToHost,
+        const size_t gs = (size_t)h->dp.gstride;
+        std::vector<unsigned long long> g(4 * gs);
+        CK(h, cudaMemcpyAsync(g.data(), h->gacc_q, sizeof(unsigned long long) * 4 * gs, cudaMemcpyDeviceToHost,
                               h->stream));
         CK(h, cudaStreamSynchronize(h->stream));
         for (size_t i = 0; i < nodes; i++) {
-            out[i] = (double)(long long)g[4 * i] * h->dp.q_inv_m;
-            for (int c = 1; c < 4; c++) out[c * nodes + i] = (double)(long long)g[4 * i + c] * h->dp.q_inv_p;
+            out[i] = (double)(long long)g[i] * h->dp.q_inv_m;
+            for (int c = 1; c < 4; c++) out[c * nodes + i] = (double)(long long)g[c * gs + i] * h->dp.q_inv_p;
         }
         return MPM_OK;
     }

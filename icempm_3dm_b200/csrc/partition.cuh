@@ -32,12 +32,13 @@ __global__ void k_halo_add_f4(float4* __restrict__ acc, long long off, int hn, c
     acc[off + i] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
 
-// The same for the fixed-point accumulator (4 int64 per node): an exact sum.
-__global__ void k_halo_add_q(unsigned long long* __restrict__ acc, long long off, int hn,
+// The same for the fixed-point accumulator (4 arrays of int64): an exact sum.
+__global__ void k_halo_add_q(unsigned long long* __restrict__ acc, long long gs, long long off, int hn,
                              const unsigned long long* __restrict__ src) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 4 * hn) return;
-    acc[4 * off + i] += src[i];
+    if (i >= hn) return;
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[c * gs + off + i] += src[(size_t)c * hn + i];
 }
 
 // One particle record of a point transfer. FP64 handles: 32 doubles (the
