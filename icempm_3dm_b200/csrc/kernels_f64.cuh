@@ -72,93 +72,137 @@ __device__ __forceinline__ bool p2g_prepare(const DevParams& P, const double* __
     return true;
 }
 
-// Calls emit(a, b, c, incM, incV) for the 27 stencil nodes (base + (a,b,c)).
-template <class Emit>
-__device__ __forceinline__ void p2g_scatter(const DevParams& P, const P2GPoint& q, Emit&& emit) {
-    double ww[3][3];
-    quad_weights<double>(q.fx, ww);
-    const double h = P.h;
+// P2G of a particle by itself, node by node, over the nodes inside the grid
+// (a stencil that leaves it raises an error: rare, and rolled).
+__device__ __forceinline__ void p2g_alone(const DevParams& P, const P2GPoint& q, double* __restrict__ grid) {
+#pragma unroll 1
+    for (int k = 0; k < 27; k++) {
+        const int o[3] = {k / 9, (k / 3) % 3, k % 3};
+        const int x = q.base[0] + o[0], y = q.base[1] + o[1], z = q.base[2] + o[2];
+        if (!node_inside(P, x, y, z)) continue;
+        double w = 1.0, d[3];
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const double dx = (a - q.fx[0]) * h;
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-            const double dy = (b - q.fx[1]) * h;
-            const double wab = ww[a][0] * ww[b][1];
-            double part[3];
-#pragma unroll
-            for (int m = 0; m < 3; m++) part[m] = q.S[m][0] * dx + q.S[m][1] * dy;
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const double dz = (c - q.fx[2]) * h;
-                const double W = wab * ww[c][2];
-                double incV[3];
-#pragma unroll
-                for (int m = 0; m < 3; m++) incV[m] = W * (q.mv[m] + (part[m] + q.S[m][2] * dz));
-                emit(a, b, c, W * q.mass, incV);
-            }
+        for (int j = 0; j < 3; j++) {
+            const double u = q.fx[j] - (double)o[j];
+            w *= o[j] == 1 ? 0.75 - u * u : 0.5 * (1.5 - fabs(u)) * (1.5 - fabs(u));
+            d[j] = -u * P.h;
         }
+        const long long ni = node_index(P, x, y, z);
+        atomicAdd(grid + ni, w * q.mass);
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            atomicAdd(grid + (r + 1) * P.gstride + ni,
+                      w * (q.mv[r] + (q.S[r][0] * d[0] + q.S[r][1] * d[1] + q.S[r][2] * d[2])));
     }
 }
 
-// Adds one node contribution to the SoA grid (4 arrays, gs doubles apart).
-__device__ __forceinline__ void grid_atomic_add(double* __restrict__ grid, long long gs, long long idx, double m,
-                                                const double v[3]) {
-    atomicAdd(grid + idx, m);
-    atomicAdd(grid + gs + idx, v[0]);
-    atomicAdd(grid + 2 * gs + idx, v[1]);
-    atomicAdd(grid + 3 * gs + idx, v[2]);
-}
-
-// Pair key of a particle: its base-cell index, or a lane-unique negative
-// value for lanes that must act alone (inactive, or a stencil reaching
-// outside the grid).
-__device__ __forceinline__ long long base_key(const DevParams& P, const P2GPoint& q, bool ok, int lane) {
-    if (!ok) return -1 - lane;
-    return node_index(P, q.base[0], q.base[1], q.base[2]);
-}
-
-// P2G with lanes that share a base cell merged in pairs by one shuffle round
-// per node (cell-sorted order puts them in neighbouring lanes; the
-// odd-ranked partner's four sums go to the even-ranked lane, which issues the
-// FP64 atomics for both), 128-thread blocks at 6 blocks per SM.
-__global__ void __launch_bounds__(128, 6) k_p2g_pairs_f64(DevParams P, const double* __restrict__ pts, size_t pitch,
-                                                             int n, double* __restrict__ grid, int* err) {
+// P2G with the sums of neighbouring lanes merged before they go to the grid.
+// In cell order (z fastest) lanes that share a base cell sit side by side:
+// the odd-ranked one's sums go to the even-ranked leader. And a leader whose
+// cell lies right above the previous leader's in z takes over (`link`) that
+// leader's sums for the two nodes of each stencil row that they share, so in
+// a chain of such cells a lane adds one node of a row instead of three.
+//
+// With the pairs alone the FP64 atomics bound the kernel (L2 and the path to
+// it at 78 %, 54.6 M RED sectors, 0.316 ms for 2 M points). The chains leave
+// 37 M sectors, and the latency of the shuffles and of the FP64 pipe becomes
+// what the time goes to: a stencil row's twelve sums are exchanged together
+// and the row ends in two predicates, at 124 registers without spills, 0.237
+// ms (64-thread blocks, 8 per SM; 10 at 96 registers: 0.242, 12 at 80: 0.245;
+// with a branch per quantity 0.279). Two points to a lane instead of the pair
+// merge (a list of slots per warp) took 0.30: no unit above 60 %, too few
+// warps for its latencies.
+constexpr int kP2GBlock = 64;
+__global__ void __launch_bounds__(kP2GBlock, 8) k_p2g_pairs_f64(DevParams P, const double* __restrict__ pts,
+                                                                  size_t pitch, int n, double* __restrict__ grid,
+                                                                  int* err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     P2GPoint q;
-    bool active = (i < n) && p2g_prepare(P, pts, pitch, i, q, err);
+    const bool active = (i < n) && p2g_prepare(P, pts, pitch, i, q, err);
     const bool inside = active && !stencil_error(P, q.base[0], q.base[1], q.base[2]);
+    if (active && !inside) p2g_alone(P, q, grid);
     if (!inside) {
         q.mass = 0;
-        if (!active) {
 #pragma unroll
-            for (int d = 0; d < 3; d++) { q.base[d] = 0; q.fx[d] = 1.0; q.mv[d] = 0; }
+        for (int d = 0; d < 3; d++) { q.base[d] = 0; q.fx[d] = 1.0; q.mv[d] = 0; }
 #pragma unroll
-            for (int r = 0; r < 3; r++)
+        for (int r = 0; r < 3; r++)
 #pragma unroll
-                for (int c = 0; c < 3; c++) q.S[r][c] = 0;
-        }
+            for (int c = 0; c < 3; c++) q.S[r][c] = 0;
     }
-    const long long key = base_key(P, q, inside, lane);
+    const int n0 = (int)node_index(P, q.base[0], q.base[1], q.base[2]);   // below 2^31: checked at creation
+    const int key = inside ? n0 : -1 - lane;
     const unsigned peers = __match_any_sync(0xffffffffu, key);
     const int rank = __popc(peers & ((1u << lane) - 1u));
-    const long long next_key = __shfl_down_sync(0xffffffffu, key, 1);
+    const int next_key = __shfl_down_sync(0xffffffffu, key, 1);
     const bool absorb = lane < 31 && next_key == key && (rank & 1) == 0;
     const bool absorbed = __shfl_up_sync(0xffffffffu, (int)absorb, 1) != 0 && lane > 0;
-    p2g_scatter(P, q, [&](int a, int b, int c, double incM, const double incV[3]) {
-        double v[4] = {incM, incV[0], incV[1], incV[2]};
+    const bool lead = inside && !absorbed;
+    const unsigned leaders = __ballot_sync(0xffffffffu, lead);
+    const unsigned lower = leaders & ((1u << lane) - 1u);
+    const unsigned upper = leaders & ~((2u << lane) - 1u);
+    const int prev = lower ? 31 - __clz(lower) : lane;
+    // key + 1 is the next node in z: a base node's z is at most Gz - 3, so it never runs into the next row
+    const int prev_key = __shfl_sync(0xffffffffu, key, prev);
+    const bool link = lead && lower && prev_key + 1 == key;
+    const unsigned links = __ballot_sync(0xffffffffu, link);
+    const bool last = lead && !(upper && ((links >> (__ffs(upper) - 1)) & 1u));   // end of its chain
+
+    double ww[3][3];
+    quad_weights<double>(q.fx, ww);
+    const double h = P.h;
+    double wdz[3];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const double o = __shfl_down_sync(0xffffffffu, v[k], 1);
-            if (absorb) v[k] += o;
+    for (int c = 0; c < 3; c++) wdz[c] = ww[c][2] * ((c - q.fx[2]) * h);
+#pragma unroll 1
+    for (int a = 0; a < 3; a++) {
+        const double wa = a == 0 ? ww[0][0] : (a == 1 ? ww[1][0] : ww[2][0]);
+        const double dx = (a - q.fx[0]) * h;
+        double pa[3];
+#pragma unroll
+        for (int r = 0; r < 3; r++) pa[r] = q.mv[r] + q.S[r][0] * dx;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const double dy = (b - q.fx[1]) * h;
+            const double wab = wa * ww[b][1];
+            double t[4][3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) t[0][c] = ww[c][2] * (wab * q.mass);
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                const double v = wab * (pa[r] + q.S[r][1] * dy), s = wab * q.S[r][2];
+#pragma unroll
+                for (int c = 0; c < 3; c++) t[r + 1][c] = ww[c][2] * v + wdz[c] * s;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const double o = __shfl_down_sync(0xffffffffu, t[k][c], 1);
+                    if (absorb) t[k][c] += o;
+                }
+#pragma unroll
+            for (int c = 2; c > 0; c--)
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const double o = __shfl_sync(0xffffffffu, t[k][c], prev);
+                    if (link) t[k][c - 1] += o;
+                }
+            double* const g = grid + (n0 + a * (int)P.slab + b * P.Gz);
+            if (lead) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) atomicAdd(g + k * P.gstride, t[k][0]);
+            }
+            if (last) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    atomicAdd(g + k * P.gstride + 1, t[k][1]);
+                    atomicAdd(g + k * P.gstride + 2, t[k][2]);
+                }
+            }
         }
-        if (!active || absorbed) return;
-        const int x = q.base[0] + a, y = q.base[1] + b, z = q.base[2] + c;
-        if (!inside && !node_inside(P, x, y, z)) return;
-        const double vv[3] = {v[1], v[2], v[3]};
-        grid_atomic_add(grid, P.gstride, node_index(P, x, y, z), v[0], vv);
-    });
+    }
 }
 
 // ----------------------------------------------------------- grid update

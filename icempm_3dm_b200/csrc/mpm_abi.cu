@@ -326,7 +326,7 @@ int launch_p2g(mpm_handle* h) {
         CK_LAUNCH(h, "p2g mixed");
         return MPM_OK;
     }
-    k_p2g_pairs_f64<<<blocks_for(n, 128), 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, n, h->grid, h->err);
+    k_p2g_pairs_f64<<<blocks_for(n, kP2GBlock), kP2GBlock, 0, h->stream>>>(h->dp, h->pts, h->pitch, n, h->grid, h->err);
     CK_LAUNCH(h, "p2g kernel");
     return MPM_OK;
 }
