@@ -157,6 +157,88 @@ int cuda_fail(mpm_handle* h, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail((h), e_, what); \
     } while (0)
 
+// The handles' device memory comes from one pool per device, so that a program
+// that makes handle after handle (a calibration makes one per evaluation, with
+// some 60 buffers) does not pay for mapping and unmapping them each time: a
+// 20,000-point gradient spent 44-52 ms, 7 of them on the device. The pool
+// keeps at most kPoolKeep bytes without an owner, returns the rest at the next
+// synchronisation, and all of it when the last handle goes while the device is
+// short of memory. Allocation and release are ordered on the handle's own
+// stream; the calls are safe from any thread.
+constexpr unsigned long long kPoolKeep = 1ull << 30;
+constexpr int kMaxDevices = 256;
+
+struct PoolTable {
+    std::mutex mu;
+    cudaMemPool_t pool[kMaxDevices] = {};
+    int handles[kMaxDevices] = {};
+};
+PoolTable& pools() {
+    static PoolTable* t = new PoolTable();   // outlives every handle, also at process exit
+    return *t;
+}
+
+cudaError_t pool_for(int device, cudaMemPool_t* out) {
+    if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
+    PoolTable& t = pools();
+    std::lock_guard<std::mutex> lock(t.mu);
+    if (!t.pool[device]) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t p = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&p, &props);
+        if (e != cudaSuccess) return e;
+        unsigned long long keep = kPoolKeep;
+        if ((e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+            cudaMemPoolDestroy(p);
+            return e;
+        }
+        t.pool[device] = p;
+    }
+    *out = t.pool[device];
+    return cudaSuccess;
+}
+
+template <class T>
+cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes) {
+    *ptr = nullptr;
+    cudaMemPool_t pool;
+    cudaError_t e = pool_for(h->device, &pool);
+    if (e != cudaSuccess) return e;
+    void* p = nullptr;
+    e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
+    if (e == cudaErrorMemoryAllocation) {   // once more without what the pool holds for nobody
+        cudaGetLastError();
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
+    }
+    if (e != cudaSuccess) return e;
+    // a caller's stream may use the memory at once
+    if (h->stream != h->own_stream && (e = cudaStreamSynchronize(h->own_stream)) != cudaSuccess) return e;
+    *ptr = static_cast<T*>(p);
+    return cudaSuccess;
+}
+
+// The work that used the memory has completed (the callers synchronise first).
+cudaError_t dev_free(mpm_handle* h, void* p) { return p ? cudaFreeAsync(p, h->own_stream) : cudaSuccess; }
+
+void pool_enter(int device) {
+    PoolTable& t = pools();
+    std::lock_guard<std::mutex> lock(t.mu);
+    t.handles[device]++;
+}
+void pool_leave(int device) {
+    PoolTable& t = pools();
+    std::lock_guard<std::mutex> lock(t.mu);
+    if (--t.handles[device] > 0 || !t.pool[device]) return;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b < total_b / 8) cudaMemPoolTrimTo(t.pool[device], 0);
+}
+
 DevParams make_dev_params(const SimParams3D& p) {
     DevParams d;
     std::memset(&d, 0, sizeof(d));
@@ -245,27 +327,31 @@ bool params_valid(const SimParams3D* p) {
 inline unsigned blocks_for(long long n, int tpb) { return (unsigned)((n + tpb - 1) / tpb); }
 
 void free_all(mpm_handle* h) {
-    cudaFree(h->pts); cudaFree(h->p0); cudaFree(h->ids); cudaFree(h->grid); cudaFree(h->sensor);
-    cudaFree(h->force_steps); cudaFree(h->force_phase); cudaFree(h->err);
-    cudaFree(h->pts_alt); cudaFree(h->p0_alt); cudaFree(h->ids_alt);
-    cudaFree(h->s_bucket); cudaFree(h->s_count); cudaFree(h->s_start); cudaFree(h->s_perm);
-    cudaFree(h->mx); cudaFree(h->p0f); cudaFree(h->gacc); cudaFree(h->gvel); cudaFree(h->gacc_q);
-    cudaFree(h->rm_list); cudaFree(h->rm_counts); cudaFree(h->xfer);
-    for (double* c : h->ckpt) cudaFree(c);
-    for (double* c : h->seg) cudaFree(c);
+    dev_free(h, h->pts); dev_free(h, h->p0); dev_free(h, h->ids); dev_free(h, h->grid); dev_free(h, h->sensor);
+    dev_free(h, h->force_steps); dev_free(h, h->force_phase); dev_free(h, h->err);
+    dev_free(h, h->pts_alt); dev_free(h, h->p0_alt); dev_free(h, h->ids_alt);
+    dev_free(h, h->s_bucket); dev_free(h, h->s_count); dev_free(h, h->s_start); dev_free(h, h->s_perm);
+    dev_free(h, h->mx); dev_free(h, h->p0f); dev_free(h, h->gacc); dev_free(h, h->gvel); dev_free(h, h->gacc_q);
+    dev_free(h, h->rm_list); dev_free(h, h->rm_counts); dev_free(h, h->xfer);
+    for (double* c : h->ckpt) dev_free(h, c);
+    for (double* c : h->seg) dev_free(h, c);
     h->ckpt.clear();
     h->seg.clear();
-    cudaFree(h->adj_A); cudaFree(h->adj_cgrad); cudaFree(h->adj_Egrad); cudaFree(h->adj_g7); cudaFree(h->adj_gb7);
-    cudaFree(h->adj_force);
-    for (double* c : h->adj_gcache) cudaFree(c);
+    dev_free(h, h->adj_A); dev_free(h, h->adj_cgrad); dev_free(h, h->adj_Egrad); dev_free(h, h->adj_g7); dev_free(h, h->adj_gb7);
+    dev_free(h, h->adj_force);
+    for (double* c : h->adj_gcache) dev_free(h, c);
     h->adj_gcache.clear();
-    cudaFree(h->adj_rmv); cudaFree(h->adj_rml); cudaFree(h->adj_rmc);
-    for (int* p : h->scan_levels) cudaFree(p);
+    dev_free(h, h->adj_rmv); dev_free(h, h->adj_rml); dev_free(h, h->adj_rmc);
+    for (int* p : h->scan_levels) dev_free(h, p);
     h->scan_levels.clear();
-    cudaFree(h->fr_f); cudaFree(h->fr_status); cudaFree(h->fr_last); cudaFree(h->fr_i); cudaFree(h->fr_rec);
-    for (int* p : h->fr_scan_levels) cudaFree(p);
+    dev_free(h, h->fr_f); dev_free(h, h->fr_status); dev_free(h, h->fr_last); dev_free(h, h->fr_i); dev_free(h, h->fr_rec);
+    for (int* p : h->fr_scan_levels) dev_free(h, p);
     h->fr_scan_levels.clear();
-    if (h->own_stream) cudaStreamDestroy(h->own_stream);
+    if (h->own_stream) {
+        cudaStreamSynchronize(h->own_stream);
+        cudaStreamDestroy(h->own_stream);
+        pool_leave(h->device);
+    }
 }
 
 size_t sensor_count(const SimParams3D& p) { return (size_t)3 * p.IndenterSubdivisions * p.GridZ; }
@@ -298,7 +384,7 @@ int mixed_from_staging(mpm_handle* h) {
                                                                   h->prms.cellsize_inv);
     CK_LAUNCH(h, "mixed from f64");
     if (h->p0) {
-        if (!h->p0f) CK(h, cudaMalloc(&h->p0f, sizeof(float) * h->pitch));
+        if (!h->p0f) CK(h, dev_alloc(h, &h->p0f, sizeof(float) * h->pitch));
         k_narrow<<<blocks_for(h->n, 256), 256, 0, h->stream>>>(h->p0, h->p0f, (int)h->n);
         CK_LAUNCH(h, "p0 narrow");
     }
@@ -453,19 +539,19 @@ int ensure_sort_scratch(mpm_handle* h) {
     const SimParams3D& p = h->prms;
     const long long nb = (long long)(p.GridXTotal + 2 * p.GridHaloSize + 1) * p.GridY * p.GridZ;
     if (nb + 1 > 0x7fffffffLL) return MPM_ERR_ARG;
-    CK(h, cudaMalloc(&h->pts_alt, sizeof(double) * MPM_N_PTS_ARRAYS * h->pitch));
-    CK(h, cudaMalloc(&h->ids_alt, sizeof(unsigned) * h->pitch));
-    CK(h, cudaMalloc(&h->s_bucket, sizeof(int) * h->pitch));
-    CK(h, cudaMalloc(&h->s_perm, sizeof(unsigned) * h->pitch));
-    CK(h, cudaMalloc(&h->s_count, sizeof(int) * (nb + 1)));
-    CK(h, cudaMalloc(&h->s_start, sizeof(int) * (nb + 1)));
+    CK(h, dev_alloc(h, &h->pts_alt, sizeof(double) * MPM_N_PTS_ARRAYS * h->pitch));
+    CK(h, dev_alloc(h, &h->ids_alt, sizeof(unsigned) * h->pitch));
+    CK(h, dev_alloc(h, &h->s_bucket, sizeof(int) * h->pitch));
+    CK(h, dev_alloc(h, &h->s_perm, sizeof(unsigned) * h->pitch));
+    CK(h, dev_alloc(h, &h->s_count, sizeof(int) * (nb + 1)));
+    CK(h, dev_alloc(h, &h->s_start, sizeof(int) * (nb + 1)));
     long long m = nb + 1;
     while (m > kScanTile) {
         m = (m + kScanTile - 1) / kScanTile;
         int* sums = nullptr;
         int* scanned = nullptr;
-        CK(h, cudaMalloc(&sums, sizeof(int) * m));
-        CK(h, cudaMalloc(&scanned, sizeof(int) * m));
+        CK(h, dev_alloc(h, &sums, sizeof(int) * m));
+        CK(h, dev_alloc(h, &scanned, sizeof(int) * m));
         h->scan_levels.push_back(sums);
         h->scan_levels.push_back(scanned);
         h->scan_sizes.push_back((int)m);
@@ -538,7 +624,7 @@ int do_sort_f64(mpm_handle* h) {
                                                                                        h->pitch, 1, h->s_perm, kept);
         CK_LAUNCH(h, "gather ids");
         if (h->p0) {
-            if (!h->p0_alt) CK(h, cudaMalloc(&h->p0_alt, sizeof(double) * h->pitch));
+            if (!h->p0_alt) CK(h, dev_alloc(h, &h->p0_alt, sizeof(double) * h->pitch));
             k_gather_rows<double><<<dim3(blocks_for(kept, 256), 1), 256, 0, h->stream>>>(h->p0, h->pitch, h->p0_alt,
                                                                                          h->pitch, 1, h->s_perm, kept);
             CK_LAUNCH(h, "gather p0");
@@ -584,8 +670,9 @@ mpm_handle* mpm_create(const SimParams3D* prms, int precision, unsigned capacity
             st = MPM_ERR_NO_DEVICE;
             break;
         }
-        cudaDeviceProp prop;
-        if (cudaGetDeviceProperties(&prop, device) != cudaSuccess || prop.major < 10) {
+        int major = 0, sms = 0;
+        if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess || major < 10 ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
             st = MPM_ERR_NO_DEVICE;
             break;
         }
@@ -596,31 +683,32 @@ mpm_handle* mpm_create(const SimParams3D* prms, int precision, unsigned capacity
         h->precision = precision;
         h->device = device;
         h->capacity = capacity;
-        h->num_sms = prop.multiProcessorCount;
+        h->num_sms = sms;
         h->pitch = ((size_t)capacity + 31) / 32 * 32;
         if (cudaSetDevice(device) != cudaSuccess) { st = MPM_ERR_CUDA; break; }
         if (cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking) != cudaSuccess) { st = MPM_ERR_CUDA; break; }
         h->stream = h->own_stream;
+        pool_enter(device);
         const size_t ns = sensor_count(*prms);
-        if (cudaMalloc(&h->pts, sizeof(double) * MPM_N_PTS_ARRAYS * h->pitch) != cudaSuccess ||
-            cudaMalloc(&h->ids, sizeof(unsigned) * h->pitch) != cudaSuccess ||
-            cudaMalloc(&h->grid, sizeof(double) * 4 * (size_t)h->dp.gstride) != cudaSuccess ||
-            cudaMalloc(&h->sensor, sizeof(double) * ns) != cudaSuccess ||
-            cudaMalloc(&h->force_phase, sizeof(double) * 3) != cudaSuccess ||
-            cudaMalloc(&h->err, sizeof(int)) != cudaSuccess) {
+        if (dev_alloc(h, &h->pts, sizeof(double) * MPM_N_PTS_ARRAYS * h->pitch) != cudaSuccess ||
+            dev_alloc(h, &h->ids, sizeof(unsigned) * h->pitch) != cudaSuccess ||
+            dev_alloc(h, &h->grid, sizeof(double) * 4 * (size_t)h->dp.gstride) != cudaSuccess ||
+            dev_alloc(h, &h->sensor, sizeof(double) * ns) != cudaSuccess ||
+            dev_alloc(h, &h->force_phase, sizeof(double) * 3) != cudaSuccess ||
+            dev_alloc(h, &h->err, sizeof(int)) != cudaSuccess) {
             st = MPM_ERR_CUDA;
             break;
         }
-        if (cudaMalloc(&h->rm_list, sizeof(int) * h->pitch) != cudaSuccess ||
-            cudaMalloc(&h->rm_counts, sizeof(int) * 2) != cudaSuccess) {
+        if (dev_alloc(h, &h->rm_list, sizeof(int) * h->pitch) != cudaSuccess ||
+            dev_alloc(h, &h->rm_counts, sizeof(int) * 2) != cudaSuccess) {
             st = MPM_ERR_CUDA;
             break;
         }
         cudaMemsetAsync(h->rm_counts, 0, sizeof(int) * 2, h->stream);
         if (precision == MPM_PRECISION_MIXED) {
-            if (cudaMalloc(&h->mx, sizeof(float) * MPM_N_PTS_ARRAYS * h->pitch) != cudaSuccess ||
-                cudaMalloc(&h->gacc, sizeof(float4) * (size_t)h->dp.nodes) != cudaSuccess ||
-                cudaMalloc(&h->gvel, sizeof(float4) * (size_t)h->dp.nodes) != cudaSuccess) {
+            if (dev_alloc(h, &h->mx, sizeof(float) * MPM_N_PTS_ARRAYS * h->pitch) != cudaSuccess ||
+                dev_alloc(h, &h->gacc, sizeof(float4) * (size_t)h->dp.nodes) != cudaSuccess ||
+                dev_alloc(h, &h->gvel, sizeof(float4) * (size_t)h->dp.nodes) != cudaSuccess) {
                 st = MPM_ERR_CUDA;
                 break;
             }
@@ -646,7 +734,11 @@ mpm_handle* mpm_create(const SimParams3D* prms, int precision, unsigned capacity
 void mpm_destroy(mpm_handle* h) {
     if (!h) return;
     cudaSetDevice(h->device);
-    cudaStreamSynchronize(h->stream);
+    // the memory goes back to the pool: nothing may still use it
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaDeviceSynchronize();
+    }
     free_all(h);
     delete h;
 }
@@ -696,17 +788,17 @@ int mpm_upload_cohesion(mpm_handle* h, const double* c, unsigned n) {
     if (!h) return MPM_ERR_ARG;
     if (!c) {
         cudaStreamSynchronize(h->stream);
-        cudaFree(h->p0);
-        cudaFree(h->p0_alt);
-        cudaFree(h->p0f);
+        dev_free(h, h->p0);
+        dev_free(h, h->p0_alt);
+        dev_free(h, h->p0f);
         h->p0 = h->p0_alt = nullptr;
         h->p0f = nullptr;
         h->p2g_ready = false;
         return MPM_OK;
     }
     if (n != h->n || h->prms.DP_tan_phi == 0) return MPM_ERR_ARG;
-    if (!h->p0) CK(h, cudaMalloc(&h->p0, sizeof(double) * h->pitch));
-    if (is_mixed(h) && !h->p0f) CK(h, cudaMalloc(&h->p0f, sizeof(float) * h->pitch));
+    if (!h->p0) CK(h, dev_alloc(h, &h->p0, sizeof(double) * h->pitch));
+    if (is_mixed(h) && !h->p0f) CK(h, dev_alloc(h, &h->p0f, sizeof(float) * h->pitch));
     h->p2g_ready = false;
     if (n == 0) return MPM_OK;
     // cohesion to the device as given, then p0 = c / tan(phi) there (the same
@@ -783,10 +875,10 @@ int mpm_set_grid_accumulation(mpm_handle* h, int mode) {
     if (!is_mixed(h)) return mode == MPM_ACCUM_FLOAT ? MPM_OK : MPM_ERR_ARG;
     CK(h, cudaStreamSynchronize(h->stream));
     if (mode == MPM_ACCUM_FIXED && !h->gacc_q) {
-        CK(h, cudaMalloc(&h->gacc_q, sizeof(unsigned long long) * 4 * (size_t)h->dp.gstride));
+        CK(h, dev_alloc(h, &h->gacc_q, sizeof(unsigned long long) * 4 * (size_t)h->dp.gstride));
         CK(h, cudaMemsetAsync(h->gacc_q, 0, sizeof(unsigned long long) * 4 * (size_t)h->dp.gstride, h->stream));
     } else if (mode == MPM_ACCUM_FLOAT && h->gacc_q) {
-        CK(h, cudaFree(h->gacc_q));
+        CK(h, dev_free(h, h->gacc_q));
         h->gacc_q = nullptr;
     }
     h->p2g_ready = false;   // the next step computes its P2G into the selected accumulator
@@ -806,18 +898,18 @@ namespace {
 int ensure_frame_scratch(mpm_handle* h) {
     if (h->fr_f) return MPM_OK;
     const size_t p = h->pitch;
-    CK(h, cudaMalloc(&h->fr_f, sizeof(float) * 7 * p));
-    CK(h, cudaMalloc(&h->fr_status, p));
-    CK(h, cudaMalloc(&h->fr_last, sizeof(int) * p));
-    CK(h, cudaMalloc(&h->fr_i, sizeof(int) * 8 * (p + 1)));
-    CK(h, cudaMalloc(&h->fr_rec, (sizeof(UpdPosRec) + sizeof(UpdJpRec) + sizeof(UpdStatusRec)) * p));
+    CK(h, dev_alloc(h, &h->fr_f, sizeof(float) * 7 * p));
+    CK(h, dev_alloc(h, &h->fr_status, p));
+    CK(h, dev_alloc(h, &h->fr_last, sizeof(int) * p));
+    CK(h, dev_alloc(h, &h->fr_i, sizeof(int) * 8 * (p + 1)));
+    CK(h, dev_alloc(h, &h->fr_rec, (sizeof(UpdPosRec) + sizeof(UpdJpRec) + sizeof(UpdStatusRec)) * p));
     long long m = (long long)p + 1;
     while (m > kScanTile) {
         m = (m + kScanTile - 1) / kScanTile;
         int* sums = nullptr;
         int* scanned = nullptr;
-        CK(h, cudaMalloc(&sums, sizeof(int) * m));
-        CK(h, cudaMalloc(&scanned, sizeof(int) * m));
+        CK(h, dev_alloc(h, &sums, sizeof(int) * m));
+        CK(h, dev_alloc(h, &scanned, sizeof(int) * m));
         h->fr_scan_levels.push_back(sums);
         h->fr_scan_levels.push_back(scanned);
     }
@@ -948,9 +1040,9 @@ int mpm_step(mpm_handle* h, int nsteps, double* force_hist) {
     if (nsteps == 0) return MPM_OK;
     if (nsteps > h->force_steps_cap) {
         CK(h, cudaStreamSynchronize(h->stream));
-        cudaFree(h->force_steps);
+        dev_free(h, h->force_steps);
         h->force_steps = nullptr;
-        CK(h, cudaMalloc(&h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
+        CK(h, dev_alloc(h, &h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
         h->force_steps_cap = nsteps;
     }
     CK(h, cudaMemsetAsync(h->force_steps, 0, sizeof(double) * 3 * (size_t)nsteps, h->stream));
@@ -1106,7 +1198,7 @@ int mpm_set_partition(mpm_handle* h, int id, int x0, int gxp, unsigned id_base) 
     h->dp.own_hi = x0 + gxp == p.GridXTotal ? p.GridXTotal + halo : x0 + gxp;
     h->dp.node_lo = (int)((long long)x0 * h->dp.slab);
     h->dp.node_hi = (int)((long long)(x0 + gxp + 2 * halo) * h->dp.slab);
-    if (!h->xfer) CK(h, cudaMalloc(&h->xfer, sizeof(int) * 3));
+    if (!h->xfer) CK(h, dev_alloc(h, &h->xfer, sizeof(int) * 3));
     return MPM_OK;
 }
 
@@ -1160,7 +1252,7 @@ int mpm_points_out(mpm_handle* h, void* left, void* right, unsigned capacity, un
                    int* max_deviation) {
     if (!h || !n_left || !n_right || (capacity && (!left || !right))) return MPM_ERR_ARG;
     if (!h->uploaded) return MPM_ERR_STATE;
-    if (!h->xfer) CK(h, cudaMalloc(&h->xfer, sizeof(int) * 3));
+    if (!h->xfer) CK(h, dev_alloc(h, &h->xfer, sizeof(int) * 3));
     CK(h, cudaMemsetAsync(h->xfer, 0, sizeof(int) * 3, h->stream));
     const SimParams3D& p = h->prms;
     XferGeom G;
@@ -1663,9 +1755,9 @@ int mpm_multi_step(mpm_multi* m, int nsteps, double* force_hist) {
         CK(h, cudaSetDevice(h->device));
         if (nsteps > h->force_steps_cap) {
             CK(h, cudaStreamSynchronize(h->stream));
-            cudaFree(h->force_steps);
+            dev_free(h, h->force_steps);
             h->force_steps = nullptr;
-            CK(h, cudaMalloc(&h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
+            CK(h, dev_alloc(h, &h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
             h->force_steps_cap = nsteps;
         }
         CK(h, cudaMemsetAsync(h->force_steps, 0, sizeof(double) * 3 * (size_t)nsteps, h->stream));
@@ -2111,37 +2203,37 @@ int ensure_adjoint_buffers(mpm_handle* h, int nsteps, int every) {
     const int nck = (nsteps + every - 1) / every;
     while ((int)h->ckpt.size() < nck) {
         double* b = nullptr;
-        CK(h, cudaMalloc(&b, state_bytes(h)));
+        CK(h, dev_alloc(h, &b, state_bytes(h)));
         h->ckpt.push_back(b);
     }
     while ((int)h->seg.size() < every + 1) {
         double* b = nullptr;
-        CK(h, cudaMalloc(&b, state_bytes(h)));
+        CK(h, dev_alloc(h, &b, state_bytes(h)));
         h->seg.push_back(b);
     }
     while ((int)h->adj_gcache.size() < every) {
         double* b = nullptr;
-        CK(h, cudaMalloc(&b, sizeof(double) * 4 * (size_t)h->dp.gstride));
+        CK(h, dev_alloc(h, &b, sizeof(double) * 4 * (size_t)h->dp.gstride));
         h->adj_gcache.push_back(b);
     }
     h->ckpt_prms.resize(nck);
     if (every > h->adj_rm_cap) {
         CK(h, cudaStreamSynchronize(h->stream));
-        cudaFree(h->adj_rml);
-        cudaFree(h->adj_rmc);
+        dev_free(h, h->adj_rml);
+        dev_free(h, h->adj_rmc);
         h->adj_rml = h->adj_rmc = nullptr;
         h->adj_rm_cap = 0;
-        CK(h, cudaMalloc(&h->adj_rml, sizeof(int) * h->pitch * (size_t)every));
-        CK(h, cudaMalloc(&h->adj_rmc, sizeof(int) * (size_t)every));
+        CK(h, dev_alloc(h, &h->adj_rml, sizeof(int) * h->pitch * (size_t)every));
+        CK(h, dev_alloc(h, &h->adj_rmc, sizeof(int) * (size_t)every));
         h->adj_rm_cap = every;
     }
     if (!h->adj_A) {
-        CK(h, cudaMalloc(&h->adj_A, sizeof(double) * ADJ_ROWS * h->pitch));
-        CK(h, cudaMalloc(&h->adj_cgrad, sizeof(double) * h->pitch));
-        CK(h, cudaMalloc(&h->adj_Egrad, sizeof(double)));
-        CK(h, cudaMalloc(&h->adj_g7, sizeof(double) * 7 * (size_t)h->dp.gstride));
-        CK(h, cudaMalloc(&h->adj_gb7, sizeof(double) * 7 * (size_t)h->dp.gstride));
-        CK(h, cudaMalloc(&h->adj_rmv, sizeof(double) * 10 * h->pitch));
+        CK(h, dev_alloc(h, &h->adj_A, sizeof(double) * ADJ_ROWS * h->pitch));
+        CK(h, dev_alloc(h, &h->adj_cgrad, sizeof(double) * h->pitch));
+        CK(h, dev_alloc(h, &h->adj_Egrad, sizeof(double)));
+        CK(h, dev_alloc(h, &h->adj_g7, sizeof(double) * 7 * (size_t)h->dp.gstride));
+        CK(h, dev_alloc(h, &h->adj_gb7, sizeof(double) * 7 * (size_t)h->dp.gstride));
+        CK(h, dev_alloc(h, &h->adj_rmv, sizeof(double) * 10 * h->pitch));
     }
     return MPM_OK;
 }
@@ -2207,9 +2299,9 @@ extern "C" int mpm_adjoint_forward(mpm_handle* h, int nsteps, int ckpt_every, do
     if (is_mixed(h)) {
         if (nsteps > h->adj_force_cap) {
             CK(h, cudaStreamSynchronize(h->stream));
-            cudaFree(h->adj_force);
+            dev_free(h, h->adj_force);
             h->adj_force = nullptr;
-            CK(h, cudaMalloc(&h->adj_force, sizeof(double) * 3 * (size_t)nsteps));
+            CK(h, dev_alloc(h, &h->adj_force, sizeof(double) * 3 * (size_t)nsteps));
             h->adj_force_cap = nsteps;
         }
         h->adj_ready = false;
@@ -2225,9 +2317,9 @@ extern "C" int mpm_adjoint_forward(mpm_handle* h, int nsteps, int ckpt_every, do
     }
     if (nsteps > h->force_steps_cap) {
         CK(h, cudaStreamSynchronize(h->stream));
-        cudaFree(h->force_steps);
+        dev_free(h, h->force_steps);
         h->force_steps = nullptr;
-        CK(h, cudaMalloc(&h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
+        CK(h, dev_alloc(h, &h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
         h->force_steps_cap = nsteps;
     }
     CK(h, cudaMemsetAsync(h->force_steps, 0, sizeof(double) * 3 * (size_t)nsteps, h->stream));
