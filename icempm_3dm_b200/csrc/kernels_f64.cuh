@@ -440,12 +440,17 @@ __device__ __forceinline__ bool g2p_advance_trial(const DevParams& P, double pos
 // partition_kernel_g2p without migration (mpm_kernels.cuh:237-351), up to
 // the failure test; a crushed point is appended to rm_list and its return map
 // runs in k_return_map_f64 (it needs the SVD, whose registers would hold every
-// thread of this kernel). 7 blocks of 128 per SM at 72 registers: 0.80 ms per
-// launch on the 8 M block against 0.90 ms with the return map inline at 128
-// registers (5 blocks: 0.90, 6: 0.85, 8 at 64 registers: 0.83 ms).
-constexpr int kG2PF64Blocks = 7;
+// thread of this kernel). Bound by the latency of the grid loads, so registers
+// decide how many of them are in flight: F and Jp_inv travel to the thread's
+// column of shared memory (cp.async, issued before the gather and read after
+// it) instead of holding 20 registers through it. 2 M points: 0.225 -> 0.212
+// ms with its return map (64-thread blocks, 14 per SM at 72 registers; 12 at
+// 80: 0.221, 16 at 64: 0.230; 7 of 128: 0.213). The warp's box of nodes in
+// shared memory as well took 0.234.
+constexpr int kG2PBlock = 64;
+constexpr int kG2PF64Blocks = 14;
 template <class K>
-__global__ void __launch_bounds__(128, kG2PF64Blocks) k_g2p_f64(DevParams P, double* __restrict__ pts, size_t pitch,
+__global__ void __launch_bounds__(kG2PBlock, kG2PF64Blocks) k_g2p_f64(DevParams P, double* __restrict__ pts, size_t pitch,
                                                  int n, const double* __restrict__ grid, int record_pq,
                                                  int* err, int* __restrict__ rm_list, int* __restrict__ rm_count) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -455,14 +460,21 @@ __global__ void __launch_bounds__(128, kG2PF64Blocks) k_g2p_f64(DevParams P, dou
     double pos[3], F[3][3];
 #pragma unroll
     for (int d = 0; d < 3; d++) pos[d] = pts[(MPM_POSX + d) * pitch + i];
+    __shared__ double fs[10 * kG2PBlock];
+    const unsigned fdst = (unsigned)__cvta_generic_to_shared(fs + threadIdx.x);
+#pragma unroll
+    for (int q = 0; q < 10; q++)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
+                     :: "r"(fdst + 8 * kG2PBlock * q), "l"(pts + (q < 9 ? MPM_FE00 + q : MPM_IDX_JP_INV) * pitch + i) : "memory");
+    double vel[3], C[3][3];
+    g2p_gather(P, grid, pos, vel, C, err);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    const volatile double* fv = fs + threadIdx.x;
 #pragma unroll
     for (int r = 0; r < 3; r++)
 #pragma unroll
-        for (int c = 0; c < 3; c++) F[r][c] = pts[(MPM_FE00 + 3 * r + c) * pitch + i];
-    double Jp_inv = pts[MPM_IDX_JP_INV * pitch + i];
-
-    double vel[3], C[3][3];
-    g2p_gather(P, grid, pos, vel, C, err);
+        for (int c = 0; c < 3; c++) F[r][c] = fv[(3 * r + c) * kG2PBlock];
+    double Jp_inv = fv[9 * kG2PBlock];
     double p_tr, q_tr;
     if (g2p_advance_trial(P, pos, vel, C, F, Jp_inv, util, p_tr, q_tr)) rm_list[atomicAdd(rm_count, 1)] = i;
 

@@ -485,7 +485,7 @@ int launch_g2p(mpm_handle* h, int record_pq, int* list = nullptr, int* count = n
         int r = launch_g2p2g_mixed(h, 0, record_pq, 1);
         return r ? r : launch_return_map_mixed(h, 0);
     }
-    const unsigned nb = blocks_for(n, 128);
+    const unsigned nb = blocks_for(n, kG2PBlock);
     const int cur = h->rm_parity;
     if (!list) h->rm_parity ^= 1;
     int* const cnt = list ? count : h->rm_counts + cur;
@@ -494,11 +494,11 @@ int launch_g2p(mpm_handle* h, int record_pq, int* list = nullptr, int* count = n
     if (!list) list = h->rm_list;
     const int rb = h->num_sms * 4;
     if (h->precision == MPM_PRECISION_FP64) {
-        k_g2p_f64<SvdF32><<<nb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, n, h->grid, record_pq, h->err,
+        k_g2p_f64<SvdF32><<<nb, kG2PBlock, 0, h->stream>>>(h->dp, h->pts, h->pitch, n, h->grid, record_pq, h->err,
                                                     list, cnt);
         k_return_map_f64<SvdF32><<<rb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, h->p0, list, cnt, next);
     } else {
-        k_g2p_f64<SvdF64><<<nb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, n, h->grid, record_pq, h->err,
+        k_g2p_f64<SvdF64><<<nb, kG2PBlock, 0, h->stream>>>(h->dp, h->pts, h->pitch, n, h->grid, record_pq, h->err,
                                                     list, cnt);
         k_return_map_f64<SvdF64><<<rb, 128, 0, h->stream>>>(h->dp, h->pts, h->pitch, h->p0, list, cnt, next);
     }
