@@ -276,6 +276,7 @@ __device__ __forceinline__ void block_add_double(double v, double* out) {
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_adj_update_record(DevParams P, double* __restrict__ g7, double ind_x,
                                                              double ind_y) {
+    chain_wait();
     const long long idx = (long long)blockIdx.x * BLOCK + threadIdx.x;
     if (idx >= P.nodes) return;
     const long long gs = P.gstride;
@@ -344,6 +345,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_rm_vjp(DevParams P, AdjParams Q, 
                                                       const double* __restrict__ p0arr, const double* __restrict__ A,
                                                       double* __restrict__ rmv, double* __restrict__ cgrad,
                                                       double* __restrict__ Egrad) {
+    chain_wait();
     const int j = threadIdx.x & 15;
     const int m = *count;
     double eg = 0;
@@ -381,6 +383,7 @@ __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams
                                                        const double* __restrict__ g7,
                                                        const double* __restrict__ rmv, double* __restrict__ A,
                                                        double* __restrict__ gadj) {
+    chain_wait();
     const int i = blockIdx.x * BLOCK + threadIdx.x;
     const long long util = i < n ? __double_as_longlong(S0[i]) : kDisabled;
     if (!(util & kDisabled)) {
@@ -516,6 +519,7 @@ template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, const double* __restrict__ g7,
                                                         double* __restrict__ gadj, double ind_x, double ind_y,
                                                         double fb0, double fb1, double fb2) {
+    chain_wait();
     const long long idx = (long long)blockIdx.x * BLOCK + threadIdx.x;
     if (idx >= P.nodes) return;
     const long long gs = P.gstride;
@@ -600,6 +604,7 @@ template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 4) k_adj_p2g_rev(DevParams P, AdjParams Q, const double* __restrict__ S0,
                                                        size_t pitch, int n, const double* __restrict__ gadj,
                                                        double* __restrict__ A, double* __restrict__ Egrad) {
+    chain_wait();
     const int i = blockIdx.x * BLOCK + threadIdx.x;
     double eg = 0;
     const long long util = i < n ? __double_as_longlong(S0[i]) : kDisabled;

@@ -47,6 +47,15 @@ struct DevParams {
     int node_lo, node_hi;          // node indices the update covers: slabs x0 - halo .. x0 + gxp + halo
 };
 
+// Start of every kernel of the substep: the launches carry the programmatic
+// serialisation attribute, so a kernel's blocks may be placed while the last
+// blocks of the one before it still run; they wait here until it has finished
+// and its writes are visible, and let the kernel after this one be placed.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // q = n / d and r = n % d for 0 <= n < 2^31 with the double reciprocal of d:
 // the product is within 2^-22 of n/d, so one correction step makes it exact.
 __device__ __forceinline__ long long div_by64(long long n, int d, double inv_d, int& r) {

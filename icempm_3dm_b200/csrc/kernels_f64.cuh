@@ -116,6 +116,7 @@ constexpr int kP2GBlock = 64;
 __global__ void __launch_bounds__(kP2GBlock, 8) k_p2g_pairs_f64(DevParams P, const double* __restrict__ pts,
                                                                   size_t pitch, int n, double* __restrict__ grid,
                                                                   int* err) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     P2GPoint q;
@@ -291,6 +292,7 @@ constexpr int kUpdateF64NodesPerThread = 2;
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* __restrict__ grid, double ind_x, double ind_y,
                                                       double* __restrict__ sensor, double* __restrict__ force3) {
+    chain_wait();
     constexpr int NPT = kUpdateF64NodesPerThread;
     const long long idx0 = (long long)P.node_lo + (long long)blockIdx.x * (BLOCK * NPT) + threadIdx.x;
     double f[3] = {0, 0, 0};
@@ -453,6 +455,7 @@ template <class K>
 __global__ void __launch_bounds__(kG2PBlock, kG2PF64Blocks) k_g2p_f64(DevParams P, double* __restrict__ pts, size_t pitch,
                                                  int n, const double* __restrict__ grid, int record_pq,
                                                  int* err, int* __restrict__ rm_list, int* __restrict__ rm_count) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     long long util = __double_as_longlong(pts[i]);
@@ -507,6 +510,7 @@ __global__ void __launch_bounds__(128) k_return_map_f64(DevParams P, double* __r
                                                         const double* __restrict__ p0_arr,
                                                         const int* __restrict__ rm_list, const int* __restrict__ count,
                                                         int* __restrict__ next_count) {
+    chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) *next_count = 0;
     const int m = *count;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {

@@ -560,6 +560,7 @@ __device__ __forceinline__ void load_mixed(const MixedState& s, int i, int X[3],
 template <class Acc>
 __global__ void __launch_bounds__(128) k_p2g_mixed(DevParams P, MixedState s, int n, Acc acc,
                                                    int* err) {
+    chain_wait();
     __shared__ float wx_slots[3 * 128];
     const WxSlot wx{wx_slots + threadIdx.x};
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -777,6 +778,7 @@ template <class Acc>
 __global__ void __launch_bounds__(kFusedBlock, 1024 / kFusedBlock) k_g2p2g_mixed(
     DevParams P, MixedState s, int n, const float4* __restrict__ vel, Acc acc, int do_p2g,
     int record_pq, int store_vc, int* err, int* __restrict__ rm_list, int* __restrict__ rm_count) {
+    chain_wait();
     extern __shared__ __align__(128) float mixed_tile[];
     __shared__ float wx_slots[3 * 128];
     const WxSlot wx{wx_slots + threadIdx.x};
@@ -794,6 +796,7 @@ template <class Acc>
 __global__ void __launch_bounds__(128) k_return_map_mixed(DevParams P, MixedState s, const int* __restrict__ rm_list,
                                                           const int* __restrict__ count, int* __restrict__ next_count,
                                                           Acc acc, int do_p2g, int* err) {
+    chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) *next_count = 0;
     const int m = *count;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
@@ -930,6 +933,7 @@ template <int BLOCK, class Acc, int NPT = kUpdateNodesPerThread>
 __global__ void __launch_bounds__(BLOCK) k_update_mixed(DevParams P, Acc acc, float4* __restrict__ vel,
                                                         double ind_x, double ind_y, double* __restrict__ sensor,
                                                         double* __restrict__ force3) {
+    chain_wait();
     const int idx0 = P.node_lo + blockIdx.x * (BLOCK * NPT) + threadIdx.x;   // the handle keeps nodes < 2^31
     double f[3] = {0, 0, 0};
     decltype(load_node(acc, 0)) r[NPT];
