@@ -268,59 +268,6 @@ __device__ __forceinline__ void block_add_double(double v, double* out) {
     }
 }
 
-// -------------------------------------------------- node update (recording)
-
-// The node update of k_update_f64 for the reverse sweep: reads m and P
-// (arrays 0..3 of a 7-array grid), writes the final velocity to arrays 4..6
-// and leaves the momentum in place.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_adj_update_record(DevParams P, double* __restrict__ g7, double ind_x,
-                                                             double ind_y) {
-    chain_wait();
-    const long long idx = (long long)blockIdx.x * BLOCK + threadIdx.x;
-    if (idx >= P.nodes) return;
-    const long long gs = P.gstride;
-    const double mass = g7[idx];
-    double v[3] = {0, 0, 0};
-    if (mass != 0) {
-        v[0] = g7[gs + idx] / mass;
-        v[1] = g7[2 * gs + idx] / mass;
-        v[2] = g7[3 * gs + idx] / mass;
-        const int idx_z = (int)(idx % P.Gz), idx_y = (int)((idx / P.Gz) % P.Gy), idx_x = (int)(idx / P.slab);
-        const int gx = idx_x - P.halo, gy = idx_y, gz = idx_z;
-        v[1] -= P.dt_gravity;
-        const double vsq = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-        if (vsq > P.vmax_sq) {
-            const double nv = sqrt(vsq);
-            for (int k = 0; k < 3; k++) v[k] = v[k] / nv * P.vmax;
-        }
-        if (P.setup_type != 2) {
-            double n0 = gx * P.h - ind_x, n1 = gy * P.h - ind_y;
-            const double nsq = n0 * n0 + n1 * n1;
-            if (nsq < P.ind_rsq) {
-                if (nsq > 0) { const double nn = sqrt(nsq); n0 /= nn; n1 /= nn; }
-                const double vn = (v[0] - P.ind_velocity) * n0 + v[1] * n1;
-                if (vn < 0) { v[0] -= n0 * vn; v[1] -= n1 * vn; }
-            }
-        }
-        if (P.setup_type != 2) {
-            if (gy <= 2) { v[0] = v[1] = v[2] = 0; }
-        } else {
-            if (gy <= 2 && v[1] < 0) v[1] = 0;
-        }
-        if (gy >= P.Gy - 3 && v[1] > 0) v[1] = 0;
-        if (gx <= 2 && v[0] < 0) v[0] = 0;
-        else if (gx >= P.Gx - 3 && v[0] > 0) v[0] = 0;
-        if (gz <= 2 && v[2] < 0) v[2] = 0;
-        else if (gz >= P.Gz - 3 && v[2] > 0) v[2] = 0;
-        if (P.setup_type == 2 && P.drag != 0)
-            for (int k = 0; k < 3; k++) v[k] *= (1 - P.drag);
-    }
-    g7[4 * gs + idx] = v[0];
-    g7[5 * gs + idx] = v[1];
-    g7[6 * gs + idx] = v[2];
-}
-
 // ----------------------------------------------------------- reverse G2P
 
 struct AdjParams {
@@ -516,7 +463,7 @@ __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams
 // ---------------------------------------------------------- reverse node
 
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, const double* __restrict__ g7,
+__global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, double* __restrict__ g7,
                                                         double* __restrict__ gadj, double ind_x, double ind_y,
                                                         double fb0, double fb1, double fb2) {
     chain_wait();
@@ -591,6 +538,10 @@ __global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, const doubl
             Pb[k] = vb1[k] / mass;
             mb -= vb1[k] * Pm[k] / (mass * mass);
         }
+        // both are summed into again: the sums by a later segment's P2G, the
+        // velocity adjoints by the next substep's reverse G2P
+        for (int k = 0; k < 4; k++) g7[k * gs + idx] = 0.0;
+        for (int k = 0; k < 3; k++) gadj[k * gs + idx] = 0.0;
     }
     gadj[3 * gs + idx] = mb;
     gadj[4 * gs + idx] = Pb[0];

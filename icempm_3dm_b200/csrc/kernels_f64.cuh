@@ -214,8 +214,7 @@ __global__ void __launch_bounds__(kP2GBlock, 8) k_p2g_pairs_f64(DevParams P, con
 // force3 receives the block-reduced force of this substep (3 doubles).
 // One node with mass of partition_kernel_update_nodes: v (the node's momentum
 // on entry) becomes its velocity; the contact force goes to f and the sensor.
-__device__ __forceinline__ void update_node_f64(const DevParams& P, double* __restrict__ grid, long long idx,
-                                                double mass, double v[3], double ind_x, double ind_y,
+__device__ __forceinline__ void update_node_f64(const DevParams& P, double* vel, long long idx, double mass, double v[3], double ind_x, double ind_y,
                                                 double* __restrict__ sensor, double f[3]) {
     int idx_z, idx_y;
     const long long col = div_by64(idx, P.Gz, P.inv_gz, idx_z);
@@ -276,9 +275,9 @@ __device__ __forceinline__ void update_node_f64(const DevParams& P, double* __re
 #pragma unroll
         for (int k = 0; k < 3; k++) v[k] *= (1 - P.drag);
     }
-    grid[P.gstride + idx] = v[0];
-    grid[2 * P.gstride + idx] = v[1];
-    grid[3 * P.gstride + idx] = v[2];
+    vel[idx] = v[0];
+    vel[P.gstride + idx] = v[1];
+    vel[2 * P.gstride + idx] = v[2];
 }
 
 // partition_kernel_update_nodes (mpm_kernels.cuh:138-232) for one partition:
@@ -288,9 +287,17 @@ __device__ __forceinline__ void update_node_f64(const DevParams& P, double* __re
 // nodes per thread, BLOCK apart, with all eight of their sums loaded before
 // either is used (8 M block: 0.053 ms against 0.073 ms for one node per thread
 // that read a node's momentum only after its mass).
+//
+// Where the velocities (3 arrays gstride apart) go and what becomes of the sums:
+//   kVelInPlace  over the momentum; the grid holds m and v afterwards
+//   kVelClear    to another buffer; the sums are cleared for the next P2G
+//                (no clearing pass of its own between the substeps)
+//   kVelRecord   to another buffer, zero where there is no mass; the sums stay
+//                (the reverse sweep reads both)
+enum { kVelInPlace = 0, kVelClear = 1, kVelRecord = 2 };
 constexpr int kUpdateF64NodesPerThread = 2;
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* __restrict__ grid, double ind_x, double ind_y,
+template <int BLOCK, int MODE>
+__global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* grid, double* vel, double ind_x, double ind_y,
                                                       double* __restrict__ sensor, double* __restrict__ force3) {
     chain_wait();
     constexpr int NPT = kUpdateF64NodesPerThread;
@@ -308,8 +315,19 @@ __global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* __res
         }
     }
 #pragma unroll
-    for (int j = 0; j < NPT; j++)
-        if (m[j] != 0) update_node_f64(P, grid, idx0 + j * BLOCK, m[j], v[j], ind_x, ind_y, sensor, f);
+    for (int j = 0; j < NPT; j++) {
+        const long long idx = idx0 + j * BLOCK;
+        if (MODE == kVelClear && idx < P.node_hi && ((m[j] != 0) | (v[j][0] != 0) | (v[j][1] != 0) | (v[j][2] != 0))) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) grid[k * P.gstride + idx] = 0.0;
+        }
+        if (m[j] != 0) {
+            update_node_f64(P, vel, idx, m[j], v[j], ind_x, ind_y, sensor, f);
+        } else if (MODE == kVelRecord && idx < P.node_hi) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) vel[k * P.gstride + idx] = 0.0;
+        }
+    }
     // block reduction of the substep force (only blocks that touch the
     // indenter contribute non-zero values)
     __shared__ double red[3][BLOCK / 32];
@@ -335,6 +353,7 @@ __global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* __res
 
 // Gathers v and C (APIC "Bp") of one particle from the updated grid
 // (mpm_kernels.cuh:278-305). Out-of-grid nodes contribute nothing.
+// grid: 4 arrays gstride apart, the node velocities in arrays 1-3 (array 0 is not read).
 __device__ __forceinline__ void g2p_gather(const DevParams& P, const double* __restrict__ grid, const double pos[3],
                                            double vel[3], double C[3][3], int* err) {
     int base[3];
@@ -451,15 +470,21 @@ __device__ __forceinline__ bool g2p_advance_trial(const DevParams& P, double pos
 // shared memory as well took 0.234.
 constexpr int kG2PBlock = 64;
 constexpr int kG2PF64Blocks = 14;
-template <class K>
-__global__ void __launch_bounds__(kG2PBlock, kG2PF64Blocks) k_g2p_f64(DevParams P, double* __restrict__ pts, size_t pitch,
-                                                 int n, const double* __restrict__ grid, int record_pq,
-                                                 int* err, int* __restrict__ rm_list, int* __restrict__ rm_count) {
+// APART: the state is read from src and written to the rows of out (one pitch);
+// else in place on out (a second pointer costs this kernel 8 %: 72 registers).
+template <bool APART>
+__global__ void __launch_bounds__(kG2PBlock, kG2PF64Blocks) k_g2p_f64(
+    DevParams P, const double* __restrict__ src, double* __restrict__ out, size_t pitch, int n, const double* __restrict__ grid, int record_pq, int* err,
+    int* __restrict__ rm_list, int* __restrict__ rm_count) {
     chain_wait();
+    const double* const pts = APART ? src : out;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     long long util = __double_as_longlong(pts[i]);
-    if (util & kDisabled) return;
+    if (util & kDisabled) {
+        if (APART) out[i] = __longlong_as_double(util);
+        return;
+    }
     double pos[3], F[3][3];
 #pragma unroll
     for (int d = 0; d < 3; d++) pos[d] = pts[(MPM_POSX + d) * pitch + i];
@@ -483,21 +508,21 @@ __global__ void __launch_bounds__(kG2PBlock, kG2PF64Blocks) k_g2p_f64(DevParams 
 
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        pts[(MPM_POSX + d) * pitch + i] = pos[d];
-        pts[(MPM_VELX + d) * pitch + i] = vel[d];
+        out[(MPM_POSX + d) * pitch + i] = pos[d];
+        out[(MPM_VELX + d) * pitch + i] = vel[d];
     }
 #pragma unroll
     for (int r = 0; r < 3; r++)
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            pts[(MPM_FE00 + 3 * r + c) * pitch + i] = F[r][c];
-            pts[(MPM_BP00 + 3 * r + c) * pitch + i] = C[r][c];
+            out[(MPM_FE00 + 3 * r + c) * pitch + i] = F[r][c];
+            out[(MPM_BP00 + 3 * r + c) * pitch + i] = C[r][c];
         }
-    pts[MPM_IDX_JP_INV * pitch + i] = Jp_inv;
-    pts[i] = __longlong_as_double(util);
+    out[MPM_IDX_JP_INV * pitch + i] = Jp_inv;
+    out[i] = __longlong_as_double(util);
     if (record_pq) {
-        pts[MPM_IDX_P * pitch + i] = p_tr;
-        pts[MPM_IDX_Q * pitch + i] = q_tr;
+        out[MPM_IDX_P * pitch + i] = p_tr;
+        out[MPM_IDX_Q * pitch + i] = q_tr;
     }
 }
 

@@ -66,6 +66,7 @@ struct mpm_handle {
     double* p0 = nullptr;             // per-particle apex shift (optional)
     unsigned* ids = nullptr;          // upload index of each particle
     double* grid = nullptr;           // AoS {m, mv} per node
+    double* gvel64 = nullptr;         // FP64 node velocities between the substeps of a call (arrays 1-3 of 4 x gstride)
     double* sensor = nullptr;         // 3 * subdiv * Gz
     double* force_steps = nullptr;    // 3 per substep of the running mpm_step
     int force_steps_cap = 0;
@@ -106,13 +107,12 @@ struct mpm_handle {
     double* adj_A = nullptr;          // ADJ_ROWS x pitch particle adjoints
     double* adj_cgrad = nullptr;      // dL/dc per particle
     double* adj_Egrad = nullptr;      // dL/dE
-    double* adj_g7 = nullptr;         // recomputed grid: m, P, final v (7 x gstride)
     double* adj_gb7 = nullptr;        // grid adjoints: vb, mb, Pb (7 x gstride)
     int adj_steps = 0, adj_every = 0;
     bool adj_ready = false;
     double* adj_force = nullptr;      // force history of a mixed adjoint forward (3 per substep)
     int adj_force_cap = 0;
-    std::vector<double*> adj_gcache;  // P2G grid of each substep of the segment being reversed
+    std::vector<double*> adj_gcache;  // grid of each substep of the segment being reversed: m, P, v (7 x gstride)
     double* adj_rmv = nullptr;        // return-map VJP of the crushed points (10 x pitch)
     int* adj_rml = nullptr;           // crushed points of each substep of the segment (pitch per substep)
     int* adj_rmc = nullptr;           // and their counts
@@ -327,7 +327,7 @@ bool params_valid(const SimParams3D* p) {
 inline unsigned blocks_for(long long n, int tpb) { return (unsigned)((n + tpb - 1) / tpb); }
 
 void free_all(mpm_handle* h) {
-    dev_free(h, h->pts); dev_free(h, h->p0); dev_free(h, h->ids); dev_free(h, h->grid); dev_free(h, h->sensor);
+    dev_free(h, h->pts); dev_free(h, h->p0); dev_free(h, h->ids); dev_free(h, h->grid); dev_free(h, h->gvel64); dev_free(h, h->sensor);
     dev_free(h, h->force_steps); dev_free(h, h->force_phase); dev_free(h, h->err);
     dev_free(h, h->pts_alt); dev_free(h, h->p0_alt); dev_free(h, h->ids_alt);
     dev_free(h, h->s_bucket); dev_free(h, h->s_count); dev_free(h, h->s_start); dev_free(h, h->s_perm);
@@ -337,7 +337,7 @@ void free_all(mpm_handle* h) {
     for (double* c : h->seg) dev_free(h, c);
     h->ckpt.clear();
     h->seg.clear();
-    dev_free(h, h->adj_A); dev_free(h, h->adj_cgrad); dev_free(h, h->adj_Egrad); dev_free(h, h->adj_g7); dev_free(h, h->adj_gb7);
+    dev_free(h, h->adj_A); dev_free(h, h->adj_cgrad); dev_free(h, h->adj_Egrad); dev_free(h, h->adj_gb7);
     dev_free(h, h->adj_force);
     for (double* c : h->adj_gcache) dev_free(h, c);
     h->adj_gcache.clear();
@@ -421,7 +421,8 @@ void chain(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem,
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-int launch_p2g(mpm_handle* h) {
+// FP64 modes: src and acc, the particle rows and the grid sums (default: the handle's own).
+int launch_p2g(mpm_handle* h, const double* src = nullptr, double* acc = nullptr) {
     const int n = (int)h->n;
     if (n == 0) return MPM_OK;
     if (is_mixed(h)) {
@@ -432,12 +433,15 @@ int launch_p2g(mpm_handle* h) {
         CK_LAUNCH(h, "p2g mixed");
         return MPM_OK;
     }
-    chain(k_p2g_pairs_f64, blocks_for(n, kP2GBlock), kP2GBlock, 0, h->stream, h->dp, h->pts, h->pitch, n, h->grid, h->err);
+    chain(k_p2g_pairs_f64, blocks_for(n, kP2GBlock), kP2GBlock, 0, h->stream, h->dp, src ? src : h->pts, h->pitch, n,
+          acc ? acc : h->grid, h->err);
     CK_LAUNCH(h, "p2g kernel");
     return MPM_OK;
 }
 
-int launch_update(mpm_handle* h, double ind_x, double ind_y, double* force3) {
+// FP64 modes: mode kVelInPlace works on the handle's grid, the others on acc and vel.
+int launch_update(mpm_handle* h, double ind_x, double ind_y, double* force3, int mode = kVelInPlace,
+                  double* acc = nullptr, double* vel = nullptr) {
     // the nodes of the partition's window (one partition: the whole grid), two per thread
     if (is_mixed(h)) {
         const unsigned nbm = blocks_for((long long)h->dp.node_hi - h->dp.node_lo, 256 * kUpdateNodesPerThread);
@@ -450,7 +454,14 @@ int launch_update(mpm_handle* h, double ind_x, double ind_y, double* force3) {
         CK_LAUNCH(h, "update mixed");
         return MPM_OK;
     }
-    chain(k_update_f64<256>, blocks_for((long long)h->dp.node_hi - h->dp.node_lo, 256 * kUpdateF64NodesPerThread), 256, 0, h->stream, h->dp, h->grid, ind_x, ind_y, h->sensor, force3);
+    const unsigned nb = blocks_for((long long)h->dp.node_hi - h->dp.node_lo, 256 * kUpdateF64NodesPerThread);
+    if (mode == kVelInPlace)
+        chain(k_update_f64<256, kVelInPlace>, nb, 256, 0, h->stream, h->dp, h->grid, h->grid + h->dp.gstride, ind_x,
+              ind_y, h->sensor, force3);
+    else if (mode == kVelClear)
+        chain(k_update_f64<256, kVelClear>, nb, 256, 0, h->stream, h->dp, acc, vel, ind_x, ind_y, h->sensor, force3);
+    else
+        chain(k_update_f64<256, kVelRecord>, nb, 256, 0, h->stream, h->dp, acc, vel, ind_x, ind_y, h->sensor, force3);
     CK_LAUNCH(h, "update kernel");
     return MPM_OK;
 }
@@ -492,9 +503,12 @@ int launch_g2p2g_mixed(mpm_handle* h, int do_p2g, int record_pq, int store_vc) {
     return MPM_OK;
 }
 
-// list, count (FP64 modes, may be null): where the crushed points are listed
-// (count zeroed by the caller) instead of the handle's own list.
-int launch_g2p(mpm_handle* h, int record_pq, int* list = nullptr, int* count = nullptr) {
+// FP64 modes, each may be null: grid the node velocities in arrays 1-3 (default:
+// the handle's grid after an update in place), src and out the particle rows read and
+// written (default: the handle's), list and count where the crushed points are
+// listed (count zeroed by the caller) instead of the handle's own list.
+int launch_g2p(mpm_handle* h, int record_pq, const double* grid = nullptr, const double* src = nullptr,
+               double* out = nullptr, int* list = nullptr, int* count = nullptr) {
     const int n = (int)h->n;
     if (n == 0) return MPM_OK;
     if (is_mixed(h)) {
@@ -509,15 +523,18 @@ int launch_g2p(mpm_handle* h, int record_pq, int* list = nullptr, int* count = n
     int* const next = h->rm_counts + (list ? cur : cur ^ 1);
     if (!list) list = h->rm_list;
     const int rb = h->num_sms * 4;
-    if (h->precision == MPM_PRECISION_FP64) {
-        chain(k_g2p_f64<SvdF32>, nb, kG2PBlock, 0, h->stream, h->dp, h->pts, h->pitch, n, h->grid, record_pq, h->err,
-                                                    list, cnt);
-        chain(k_return_map_f64<SvdF32>, rb, 128, 0, h->stream, h->dp, h->pts, h->pitch, h->p0, list, cnt, next);
-    } else {
-        chain(k_g2p_f64<SvdF64>, nb, kG2PBlock, 0, h->stream, h->dp, h->pts, h->pitch, n, h->grid, record_pq, h->err,
-                                                    list, cnt);
-        chain(k_return_map_f64<SvdF64>, rb, 128, 0, h->stream, h->dp, h->pts, h->pitch, h->p0, list, cnt, next);
-    }
+    if (!grid) grid = h->grid;
+    if (out)
+        chain(k_g2p_f64<true>, nb, kG2PBlock, 0, h->stream, h->dp, src, out, h->pitch, n, grid, record_pq, h->err, list,
+              cnt);
+    else
+        chain(k_g2p_f64<false>, nb, kG2PBlock, 0, h->stream, h->dp, nullptr, h->pts, h->pitch, n, grid, record_pq,
+              h->err, list, cnt);
+    if (!out) out = h->pts;
+    if (h->precision == MPM_PRECISION_FP64)
+        chain(k_return_map_f64<SvdF32>, rb, 128, 0, h->stream, h->dp, out, h->pitch, h->p0, list, cnt, next);
+    else
+        chain(k_return_map_f64<SvdF64>, rb, 128, 0, h->stream, h->dp, out, h->pitch, h->p0, list, cnt, next);
     CK_LAUNCH(h, "g2p kernel");
     return MPM_OK;
 }
@@ -540,6 +557,30 @@ int reset_grid(mpm_handle* h) {
     for (int c = 0; c < 4; c++)
         CK(h, cudaMemsetAsync(h->grid + c * h->dp.gstride + h->dp.node_lo, 0, sizeof(double) * cnt, h->stream));
     return MPM_OK;
+}
+
+// P2G, node update and G2P of substep s of a run of nsteps (FP64 modes). Between
+// the substeps the update itself clears the sums, so only the first one clears
+// the grid; the last leaves m and v in it, as the phase calls do.
+int fp64_grid_step(mpm_handle* h, int s, int nsteps, double* force3) {
+    const SimParams3D& p = h->prms;
+    int r;
+    const bool last = s == nsteps - 1;
+    if (!last && !h->gvel64) {
+        const size_t bytes = sizeof(double) * 4 * (size_t)h->dp.gstride;
+        CK(h, dev_alloc(h, &h->gvel64, bytes));
+        CK(h, cudaMemsetAsync(h->gvel64, 0, bytes, h->stream));
+    }
+    if (s == 0 && (r = reset_grid(h))) return r;
+    if ((r = launch_p2g(h))) return r;
+    const int record = (p.SimulationStep % p.UpdateEveryNthStep) == 0;
+    if (last) {
+        if ((r = launch_update(h, p.indenter_x, p.indenter_y, force3))) return r;
+        return launch_g2p(h, record);
+    }
+    if ((r = launch_update(h, p.indenter_x, p.indenter_y, force3, kVelClear, h->grid,
+                           h->gvel64 + h->dp.gstride))) return r;
+    return launch_g2p(h, record, h->gvel64);
 }
 
 int read_error(mpm_handle* h, int* code) {
@@ -1087,11 +1128,7 @@ int mpm_step(mpm_handle* h, int nsteps, double* force_hist) {
             }
             continue;
         }
-        if ((r = reset_grid(h))) return r;
-        if ((r = launch_p2g(h))) return r;
-        if ((r = launch_update(h, p.indenter_x, p.indenter_y, h->force_steps + 3 * s))) return r;
-        const int record = (p.SimulationStep % p.UpdateEveryNthStep) == 0;
-        if ((r = launch_g2p(h, record))) return r;
+        if ((r = fp64_grid_step(h, s, nsteps, h->force_steps + 3 * s))) return r;
         p.SimulationStep += 1;
         if (h->sort_interval > 0 && ++h->steps_since_sort >= h->sort_interval) {
             if ((r = do_sort(h))) return r;
@@ -2194,23 +2231,26 @@ namespace {
 
 size_t state_bytes(const mpm_handle* h) { return sizeof(double) * MPM_N_PTS_ARRAYS * h->pitch; }
 
-// One FP64 substep of Model3D::Step on the particle rows at h->pts;
-// p2g_copy (may be null) receives the grid after P2G (4 x gstride doubles),
-// rm_list and rm_count (zeroed) the points that it crushed.
-int fp64_substep(mpm_handle* h, double* force3, double* p2g_copy = nullptr, int* rm_list = nullptr,
-                 int* rm_count = nullptr) {
+// The indenter's position for the next substep.
+void advance_indenter(mpm_handle* h) {
     SimParams3D& p = h->prms;
     p.SimulationTime += p.InitialTimeStep;
     p.indenter_x = p.indenter_x_initial + p.SimulationTime * p.IndVelocity;
+}
+
+// One recomputed FP64 substep of Model3D::Step, from the particle rows src to
+// the rows out: the sums and velocities stay in the 7 arrays of g7 (m, P, v;
+// the sums zero on entry), the points that it crushed in rm_list and rm_count
+// (zeroed).
+int fp64_recompute(mpm_handle* h, const double* src, double* out, double* g7, int* rm_list, int* rm_count) {
+    SimParams3D& p = h->prms;
+    advance_indenter(h);
+    double* const vgrid = g7 + 3 * h->dp.gstride;   // its arrays 1-3: arrays 4-6 of g7
     int r;
-    if ((r = reset_grid(h))) return r;
-    if ((r = launch_p2g(h))) return r;
-    if (p2g_copy)
-        CK(h, cudaMemcpyAsync(p2g_copy, h->grid, sizeof(double) * 4 * (size_t)h->dp.gstride, cudaMemcpyDeviceToDevice,
-                              h->stream));
-    if ((r = launch_update(h, p.indenter_x, p.indenter_y, force3))) return r;
-    const int record = (p.SimulationStep % p.UpdateEveryNthStep) == 0;
-    if ((r = launch_g2p(h, record, rm_list, rm_count))) return r;
+    if ((r = launch_p2g(h, src, g7))) return r;
+    if ((r = launch_update(h, p.indenter_x, p.indenter_y, h->force_phase, kVelRecord, g7,
+                           vgrid + h->dp.gstride))) return r;
+    if ((r = launch_g2p(h, 0, vgrid, src, out, rm_list, rm_count))) return r;
     p.SimulationStep += 1;
     return MPM_OK;
 }
@@ -2222,15 +2262,16 @@ int ensure_adjoint_buffers(mpm_handle* h, int nsteps, int every) {
         CK(h, dev_alloc(h, &b, state_bytes(h)));
         h->ckpt.push_back(b);
     }
-    while ((int)h->seg.size() < every + 1) {
+    while ((int)h->seg.size() < every) {
         double* b = nullptr;
         CK(h, dev_alloc(h, &b, state_bytes(h)));
         h->seg.push_back(b);
     }
     while ((int)h->adj_gcache.size() < every) {
         double* b = nullptr;
-        CK(h, dev_alloc(h, &b, sizeof(double) * 4 * (size_t)h->dp.gstride));
+        CK(h, dev_alloc(h, &b, sizeof(double) * 7 * (size_t)h->dp.gstride));
         h->adj_gcache.push_back(b);
+        CK(h, cudaMemsetAsync(b, 0, sizeof(double) * 7 * (size_t)h->dp.gstride, h->stream));
     }
     h->ckpt_prms.resize(nck);
     if (every > h->adj_rm_cap) {
@@ -2247,7 +2288,6 @@ int ensure_adjoint_buffers(mpm_handle* h, int nsteps, int every) {
         CK(h, dev_alloc(h, &h->adj_A, sizeof(double) * ADJ_ROWS * h->pitch));
         CK(h, dev_alloc(h, &h->adj_cgrad, sizeof(double) * h->pitch));
         CK(h, dev_alloc(h, &h->adj_Egrad, sizeof(double)));
-        CK(h, dev_alloc(h, &h->adj_g7, sizeof(double) * 7 * (size_t)h->dp.gstride));
         CK(h, dev_alloc(h, &h->adj_gb7, sizeof(double) * 7 * (size_t)h->dp.gstride));
         CK(h, dev_alloc(h, &h->adj_rmv, sizeof(double) * 10 * h->pitch));
     }
@@ -2344,7 +2384,9 @@ extern "C" int mpm_adjoint_forward(mpm_handle* h, int nsteps, int ckpt_every, do
             CK(h, cudaMemcpyAsync(h->ckpt[s / ckpt_every], h->pts, state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
             h->ckpt_prms[s / ckpt_every] = h->prms;
         }
-        if ((r = fp64_substep(h, h->force_steps + 3 * s))) return r;
+        advance_indenter(h);
+        if ((r = fp64_grid_step(h, s, nsteps, h->force_steps + 3 * s))) return r;
+        h->prms.SimulationStep += 1;
     }
     if (force_hist)
         CK(h, cudaMemcpyAsync(force_hist, h->force_steps, sizeof(double) * 3 * (size_t)nsteps, cudaMemcpyDeviceToHost,
@@ -2368,7 +2410,10 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
     CK(h, cudaMemsetAsync(h->adj_A, 0, sizeof(double) * ADJ_ROWS * h->pitch, h->stream));
     CK(h, cudaMemsetAsync(h->adj_cgrad, 0, sizeof(double) * h->pitch, h->stream));
     CK(h, cudaMemsetAsync(h->adj_Egrad, 0, sizeof(double), h->stream));
-    double* const pts_final = h->pts;
+    // what the sweep sums into is zero here and left zero by k_adj_node_rev
+    CK(h, cudaMemsetAsync(h->adj_gb7, 0, sizeof(double) * 3 * gs, h->stream));
+    for (int s = 0; s < std::min(k, N); s++)
+        CK(h, cudaMemsetAsync(h->adj_gcache[s], 0, sizeof(double) * 4 * gs, h->stream));
     const SimParams3D prms_final = h->prms;
     int r = MPM_OK;
     const int nseg = (N + k - 1) / k;
@@ -2376,40 +2421,34 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
         const int s0 = j * k, s1 = std::min(N, s0 + k);
         // recompute the segment's states from its checkpoint
         std::vector<SimParams3D> sp(s1 - s0);
-        CK(h, cudaMemcpyAsync(h->seg[0], h->ckpt[j], state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
+        std::vector<const double*> S(s1 - s0 + 1);   // the state before each substep, and after the last
+        S[0] = h->ckpt[j];
         h->prms = h->ckpt_prms[j];
         CK(h, cudaMemsetAsync(h->adj_rmc, 0, sizeof(int) * (size_t)(s1 - s0), h->stream));
-        for (int s = s0; s < s1 && !r; s++) {
-            double* next = h->seg[s - s0 + 1];
-            CK(h, cudaMemcpyAsync(next, h->seg[s - s0], state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
-            h->pts = next;
-            r = fp64_substep(h, h->force_phase, h->adj_gcache[s - s0], h->adj_rml + h->pitch * (size_t)(s - s0),
-                             h->adj_rmc + (s - s0));
-            sp[s - s0] = h->prms;   // holds this substep's indenter position
+        for (int m = 0; m < s1 - s0 && !r; m++) {
+            r = fp64_recompute(h, S[m], h->seg[m], h->adj_gcache[m], h->adj_rml + h->pitch * (size_t)m,
+                               h->adj_rmc + m);
+            S[m + 1] = h->seg[m];
+            sp[m] = h->prms;   // holds this substep's indenter position
         }
-        h->pts = pts_final;
         if (r) break;
         // reverse the segment
-        for (int s = s1 - 1; s >= s0; s--) {
-            const double* Sn = h->seg[s - s0];
-            const double* Sn1 = h->seg[s - s0 + 1];
-            const double ix = sp[s - s0].indenter_x, iy = sp[s - s0].indenter_y;
-            // the substep's P2G grid, as the recompute produced it
-            CK(h, cudaMemcpyAsync(h->adj_g7, h->adj_gcache[s - s0], sizeof(double) * 4 * gs, cudaMemcpyDeviceToDevice,
-                                  h->stream));
-            chain(k_adj_update_record<256>, blocks_for(dp.nodes, 256), 256, 0, h->stream, dp, h->adj_g7, ix, iy);
-            CK(h, cudaMemsetAsync(h->adj_gb7, 0, sizeof(double) * 7 * gs, h->stream));
-            chain(k_adj_rm_vjp<128>, h->num_sms * 4, 128, 0, h->stream, dp, q, Sn, Sn1, h->pitch, h->adj_rml + h->pitch * (size_t)(s - s0), h->adj_rmc + (s - s0), h->p0,
-                h->adj_A, h->adj_rmv, h->adj_cgrad, h->adj_Egrad);
-            chain(k_adj_g2p_rev<128>, blocks_for(n, 128), 128, 0, h->stream, dp, q, Sn, Sn1, h->pitch, n, h->adj_g7,
-                                                                         h->adj_rmv, h->adj_A, h->adj_gb7);
-            chain(k_adj_node_rev<256>, blocks_for(dp.nodes, 256), 256, 0, h->stream, dp, h->adj_g7, h->adj_gb7, ix, iy, dL_dforce[3 * s], dL_dforce[3 * s + 1], dL_dforce[3 * s + 2]);
-            chain(k_adj_p2g_rev<128>, blocks_for(n, 128), 128, 0, h->stream, dp, q, Sn, h->pitch, n, h->adj_gb7, h->adj_A,
-                                                                         h->adj_Egrad);
+        for (int m = s1 - s0 - 1; m >= 0; m--) {
+            const double* dl = dL_dforce + 3 * (size_t)(s0 + m);
+            const double ix = sp[m].indenter_x, iy = sp[m].indenter_y;
+            double* const g7 = h->adj_gcache[m];
+            chain(k_adj_rm_vjp<128>, h->num_sms * 4, 128, 0, h->stream, dp, q, S[m], S[m + 1], h->pitch,
+                  h->adj_rml + h->pitch * (size_t)m, h->adj_rmc + m, h->p0, h->adj_A, h->adj_rmv, h->adj_cgrad,
+                  h->adj_Egrad);
+            chain(k_adj_g2p_rev<128>, blocks_for(n, 128), 128, 0, h->stream, dp, q, S[m], S[m + 1], h->pitch, n, g7,
+                  h->adj_rmv, h->adj_A, h->adj_gb7);
+            chain(k_adj_node_rev<256>, blocks_for(dp.nodes, 256), 256, 0, h->stream, dp, g7, h->adj_gb7, ix, iy, dl[0],
+                  dl[1], dl[2]);
+            chain(k_adj_p2g_rev<128>, blocks_for(n, 128), 128, 0, h->stream, dp, q, S[m], h->pitch, n, h->adj_gb7,
+                  h->adj_A, h->adj_Egrad);
             CK_LAUNCH(h, "adjoint kernels");
         }
     }
-    h->pts = pts_final;
     h->prms = prms_final;
     if (r) return r;
     if (dL_dcohesion && n)
