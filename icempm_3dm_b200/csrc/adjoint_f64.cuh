@@ -25,6 +25,8 @@
 // (one direction per input), so it follows every branch the forward took.
 #pragma once
 
+#include <climits>
+
 #include "device_common.cuh"
 #include "physics_f64.cuh"
 #include "svd3.cuh"
@@ -324,14 +326,51 @@ __global__ void __launch_bounds__(BLOCK) k_adj_rm_vjp(DevParams P, AdjParams Q, 
     block_add_double(eg, Egrad);
 }
 
-template <int BLOCK>
+// A particle's 27 nodes on one lane, or on three (one x-layer of nine each,
+// ten particles to a warp): a lane's nodes are one long chain of loads and
+// FP64 operations, and with few particles that chain is the kernel's time. Three
+// lanes repeat the particle's own arithmetic, which costs more once the chip is
+// full: reverse sweep over 40 substeps of 3,000 points 2.85 -> 2.47 ms, 20,000
+// 3.59 -> 3.15, 100,000 6.06 -> 6.94, 500,000 21.2 -> 28.5. Three up to 192
+// points per SM (28,416), about where the three-lane blocks fill it once.
+constexpr int kRevSplitPerSM = 192;
+struct RevLane {
+    int i, part;        // particle, x-layer (lane 0 of a particle writes its results)
+    unsigned mask;      // lanes of the particle
+    int first;          // its first lane
+};
+template <int BLOCK, int LANES>
+__device__ __forceinline__ RevLane rev_lane() {
+    if (LANES == 1) return {(int)(blockIdx.x * BLOCK + threadIdx.x), 0, 0u, 0};
+    const int lane = threadIdx.x & 31, g = lane / 3;
+    const int warp = (blockIdx.x * BLOCK + threadIdx.x) >> 5;
+    return {g < 10 ? warp * 10 + g : INT_MAX, lane - 3 * g, 7u << (3 * g), 3 * g};
+}
+// Sums v over the particle's lanes (valid on its first).
+template <int LANES>
+__device__ __forceinline__ void rev_sum(double* v, int count, const RevLane& L) {
+    if (LANES == 1) return;
+#pragma unroll
+    for (int k = 0; k < count; k++) {
+        const double b = __shfl_sync(L.mask, v[k], L.first + 1);
+        const double c = __shfl_sync(L.mask, v[k], L.first + 2);
+        v[k] = (v[k] + b) + c;
+    }
+}
+inline unsigned rev_blocks(int n, int block, int lanes) {
+    const int per = lanes == 1 ? block : block / 32 * 10;
+    return (unsigned)((n + per - 1) / per);
+}
+
+template <int BLOCK, int LANES>
 __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams Q, const double* __restrict__ S0,
                                                        const double* __restrict__ S1, size_t pitch, int n,
                                                        const double* __restrict__ g7,
                                                        const double* __restrict__ rmv, double* __restrict__ A,
                                                        double* __restrict__ gadj) {
     chain_wait();
-    const int i = blockIdx.x * BLOCK + threadIdx.x;
+    const RevLane L = rev_lane<BLOCK, LANES>();
+    const int i = L.i;
     const long long util = i < n ? __double_as_longlong(S0[i]) : kDisabled;
     if (!(util & kDisabled)) {
         const long long util1 = __double_as_longlong(S1[i]);
@@ -418,9 +457,12 @@ __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams
             for (int c = 0; c < 3; c++) Cbt[r][c] = Cb[r][c] + dt * Ab[r][c];
         }
         // gather adjoint: node velocity adjoints and x-gradients
-        double xb0[3] = {xb[0], xb[1], xb[2]};
+        double xb0[3] = {0, 0, 0};
 #pragma unroll
-        for (int a = 0; a < 3; a++)
+        for (int aa = 0; aa < 3 / LANES; aa++) {
+            const int a = LANES == 1 ? aa : L.part;
+            const double wa = LANES == 1 ? w[aa][0] : (a == 0 ? w[0][0] : (a == 1 ? w[1][0] : w[2][0]));
+            const double dwa = LANES == 1 ? dwh[aa][0] : (a == 0 ? dwh[0][0] : (a == 1 ? dwh[1][0] : dwh[2][0]));
 #pragma unroll
             for (int b = 0; b < 3; b++)
 #pragma unroll
@@ -428,9 +470,9 @@ __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams
                     const int nx = base[0] + a, ny = base[1] + b, nz = base[2] + c;
                     if (!node_inside(P, nx, ny, nz)) continue;
                     const long long ni = node_index(P, nx, ny, nz);
-                    const double wt = w[a][0] * w[b][1] * w[c][2];
-                    const double gw[3] = {dwh[a][0] * w[b][1] * w[c][2], w[a][0] * dwh[b][1] * w[c][2],
-                                          w[a][0] * w[b][1] * dwh[c][2]};
+                    const double wt = wa * w[b][1] * w[c][2];
+                    const double gw[3] = {dwa * w[b][1] * w[c][2], wa * dwh[b][1] * w[c][2],
+                                          wa * w[b][1] * dwh[c][2]};
                     const double nv[3] = {g7[4 * P.gstride + ni], g7[5 * P.gstride + ni], g7[6 * P.gstride + ni]};
                     const double dd[3] = {(a - fx[0]) * h, (b - fx[1]) * h, (c - fx[2]) * h};
                     double gsc = 0;
@@ -446,9 +488,12 @@ __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams
                         xb0[d] += gw[d] * gsc - s4 * wt * ctv;
                     }
                 }
+        }
+        rev_sum<LANES>(xb0, 3, L);
+        if (L.part != 0) return;
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            A[(ADJ_X + d) * pitch + i] = xb0[d];
+            A[(ADJ_X + d) * pitch + i] = xb[d] + xb0[d];
             A[(ADJ_V + d) * pitch + i] = 0.0;
         }
 #pragma unroll
@@ -551,12 +596,13 @@ __global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, double* __r
 
 // ----------------------------------------------------------- reverse P2G
 
-template <int BLOCK>
+template <int BLOCK, int LANES>
 __global__ void __launch_bounds__(BLOCK, 4) k_adj_p2g_rev(DevParams P, AdjParams Q, const double* __restrict__ S0,
                                                        size_t pitch, int n, const double* __restrict__ gadj,
                                                        double* __restrict__ A, double* __restrict__ Egrad) {
     chain_wait();
-    const int i = blockIdx.x * BLOCK + threadIdx.x;
+    const RevLane L = rev_lane<BLOCK, LANES>();
+    const int i = L.i;
     double eg = 0;
     const long long util = i < n ? __double_as_longlong(S0[i]) : kDisabled;
     if (!(util & kDisabled)) {
@@ -607,7 +653,10 @@ __global__ void __launch_bounds__(BLOCK, 4) k_adj_p2g_rev(DevParams P, AdjParams
             for (int d = 0; d < 3; d++) dwh[k][d] = dw[k][d] * P.h_inv;
         double xb[3] = {0, 0, 0}, sP[3] = {0, 0, 0}, Qb[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
 #pragma unroll
-        for (int a = 0; a < 3; a++)
+        for (int aa = 0; aa < 3 / LANES; aa++) {
+            const int a = LANES == 1 ? aa : L.part;
+            const double wa = LANES == 1 ? w[aa][0] : (a == 0 ? w[0][0] : (a == 1 ? w[1][0] : w[2][0]));
+            const double dwa = LANES == 1 ? dwh[aa][0] : (a == 0 ? dwh[0][0] : (a == 1 ? dwh[1][0] : dwh[2][0]));
 #pragma unroll
             for (int b = 0; b < 3; b++)
 #pragma unroll
@@ -615,9 +664,9 @@ __global__ void __launch_bounds__(BLOCK, 4) k_adj_p2g_rev(DevParams P, AdjParams
                     const int nx = base[0] + a, ny = base[1] + b, nz = base[2] + c;
                     if (!node_inside(P, nx, ny, nz)) continue;
                     const long long ni = node_index(P, nx, ny, nz);
-                    const double wt = w[a][0] * w[b][1] * w[c][2];
-                    const double gw[3] = {dwh[a][0] * w[b][1] * w[c][2], w[a][0] * dwh[b][1] * w[c][2],
-                                          w[a][0] * w[b][1] * dwh[c][2]};
+                    const double wt = wa * w[b][1] * w[c][2];
+                    const double gw[3] = {dwa * w[b][1] * w[c][2], wa * dwh[b][1] * w[c][2],
+                                          wa * w[b][1] * dwh[c][2]};
                     const double mb = gadj[3 * P.gstride + ni];
                     const double Pb[3] = {gadj[4 * P.gstride + ni], gadj[5 * P.gstride + ni], gadj[6 * P.gstride + ni]};
                     const double dd[3] = {(a - fx[0]) * h, (b - fx[1]) * h, (c - fx[2]) * h};
@@ -636,6 +685,11 @@ __global__ void __launch_bounds__(BLOCK, 4) k_adj_p2g_rev(DevParams P, AdjParams
                         xb[d] += gw[d] * g - wt * qtp;
                     }
                 }
+        }
+        rev_sum<LANES>(xb, 3, L);
+        rev_sum<LANES>(sP, 3, L);
+        rev_sum<LANES>(&Qb[0][0], 9, L);
+        if (L.part == 0) {
         // Q = m C - k tau
         double Fb[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, tb[3][3];
 #pragma unroll
@@ -662,6 +716,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_adj_p2g_rev(DevParams P, AdjParams
             A[(ADJ_F + k) * pitch + i] += Fb[k / 3][k % 3];
         }
         A[ADJ_JP * pitch + i] += Jpb;
+        }
     }
     block_add_double(eg, Egrad);
 }

@@ -2407,6 +2407,7 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
     const DevParams dp = h->dp;
     const AdjParams q = adj_params(h);
     const size_t gs = (size_t)dp.gstride;
+    const bool split = n <= kRevSplitPerSM * h->num_sms;
     CK(h, cudaMemsetAsync(h->adj_A, 0, sizeof(double) * ADJ_ROWS * h->pitch, h->stream));
     CK(h, cudaMemsetAsync(h->adj_cgrad, 0, sizeof(double) * h->pitch, h->stream));
     CK(h, cudaMemsetAsync(h->adj_Egrad, 0, sizeof(double), h->stream));
@@ -2440,12 +2441,13 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
             chain(k_adj_rm_vjp<128>, h->num_sms * 4, 128, 0, h->stream, dp, q, S[m], S[m + 1], h->pitch,
                   h->adj_rml + h->pitch * (size_t)m, h->adj_rmc + m, h->p0, h->adj_A, h->adj_rmv, h->adj_cgrad,
                   h->adj_Egrad);
-            chain(k_adj_g2p_rev<128>, blocks_for(n, 128), 128, 0, h->stream, dp, q, S[m], S[m + 1], h->pitch, n, g7,
-                  h->adj_rmv, h->adj_A, h->adj_gb7);
+            const unsigned nb = rev_blocks(n, 128, split ? 3 : 1);
+            chain(split ? k_adj_g2p_rev<128, 3> : k_adj_g2p_rev<128, 1>, nb, 128, 0, h->stream, dp, q, S[m], S[m + 1],
+                  h->pitch, n, g7, h->adj_rmv, h->adj_A, h->adj_gb7);
             chain(k_adj_node_rev<256>, blocks_for(dp.nodes, 256), 256, 0, h->stream, dp, g7, h->adj_gb7, ix, iy, dl[0],
                   dl[1], dl[2]);
-            chain(k_adj_p2g_rev<128>, blocks_for(n, 128), 128, 0, h->stream, dp, q, S[m], h->pitch, n, h->adj_gb7,
-                  h->adj_A, h->adj_Egrad);
+            chain(split ? k_adj_p2g_rev<128, 3> : k_adj_p2g_rev<128, 1>, nb, 128, 0, h->stream, dp, q, S[m], h->pitch,
+                  n, h->adj_gb7, h->adj_A, h->adj_Egrad);
             CK_LAUNCH(h, "adjoint kernels");
         }
     }
