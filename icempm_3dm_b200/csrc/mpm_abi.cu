@@ -74,7 +74,8 @@ struct mpm_handle {
     int* err = nullptr;
 
     // sort scratch (allocated on first sort)
-    double* pts_alt = nullptr;
+    double* pts_alt = nullptr;        // FP64 modes: 28 rows; mixed: one row (the utility words)
+    void* mx_alt = nullptr;           // mixed: 28 rows of 4-byte words
     double* p0_alt = nullptr;
     unsigned* ids_alt = nullptr;
     int* s_bucket = nullptr;
@@ -329,7 +330,7 @@ inline unsigned blocks_for(long long n, int tpb) { return (unsigned)((n + tpb - 
 void free_all(mpm_handle* h) {
     dev_free(h, h->pts); dev_free(h, h->p0); dev_free(h, h->ids); dev_free(h, h->grid); dev_free(h, h->gvel64); dev_free(h, h->sensor);
     dev_free(h, h->force_steps); dev_free(h, h->force_phase); dev_free(h, h->err);
-    dev_free(h, h->pts_alt); dev_free(h, h->p0_alt); dev_free(h, h->ids_alt);
+    dev_free(h, h->pts_alt); dev_free(h, h->mx_alt); dev_free(h, h->p0_alt); dev_free(h, h->ids_alt);
     dev_free(h, h->s_bucket); dev_free(h, h->s_count); dev_free(h, h->s_start); dev_free(h, h->s_perm);
     dev_free(h, h->mx); dev_free(h, h->p0f); dev_free(h, h->gacc); dev_free(h, h->gvel); dev_free(h, h->gacc_q);
     dev_free(h, h->rm_list); dev_free(h, h->rm_counts); dev_free(h, h->xfer);
@@ -596,7 +597,9 @@ int ensure_sort_scratch(mpm_handle* h) {
     const SimParams3D& p = h->prms;
     const long long nb = (long long)(p.GridXTotal + 2 * p.GridHaloSize + 1) * p.GridY * p.GridZ;
     if (nb + 1 > 0x7fffffffLL) return MPM_ERR_ARG;
-    CK(h, dev_alloc(h, &h->pts_alt, sizeof(double) * MPM_N_PTS_ARRAYS * h->pitch));
+    const bool mixed = is_mixed(h);
+    CK(h, dev_alloc(h, &h->pts_alt, sizeof(double) * (mixed ? 1 : MPM_N_PTS_ARRAYS) * h->pitch));
+    if (mixed) CK(h, dev_alloc(h, &h->mx_alt, sizeof(float) * MPM_N_PTS_ARRAYS * h->pitch));
     CK(h, dev_alloc(h, &h->ids_alt, sizeof(unsigned) * h->pitch));
     CK(h, dev_alloc(h, &h->s_bucket, sizeof(int) * h->pitch));
     CK(h, dev_alloc(h, &h->s_perm, sizeof(unsigned) * h->pitch));
@@ -635,18 +638,7 @@ int exclusive_scan(mpm_handle* h, const int* in, int* out, int n, size_t level,
     return MPM_OK;
 }
 
-int do_sort_f64(mpm_handle* h);
-
 int do_sort(mpm_handle* h) {
-    if (!is_mixed(h)) return do_sort_f64(h);
-    int r = mixed_to_staging(h);
-    if (r) return r;
-    r = do_sort_f64(h);
-    if (r) return r;
-    return mixed_from_staging(h);
-}
-
-int do_sort_f64(mpm_handle* h) {
     if (h->n == 0) return MPM_OK;
     int r = ensure_sort_scratch(h);
     if (r) return r;
@@ -660,7 +652,16 @@ int do_sort_f64(mpm_handle* h) {
     const int n = (int)h->n;
     const int nb1 = G.nb + 1;
     CK(h, cudaMemsetAsync(h->s_count, 0, sizeof(int) * nb1, h->stream));
-    k_sort_keys<<<blocks_for(n, 256), 256, 0, h->stream>>>(G, h->pts, h->pitch, n, h->s_bucket, h->s_count, h->err);
+    const bool mixed = is_mixed(h);
+    if (mixed) {
+        const MixedState m = mixed_state(h);
+        k_sort_keys<<<blocks_for(n, 256), 256, 0, h->stream>>>(
+            G, SortRowsMixed{m.X, m.status, m.pitch, p.cellsize, 1.0 / (double)(1 << kFixBits)}, n, h->s_bucket,
+            h->s_count, h->err);
+    } else {
+        k_sort_keys<<<blocks_for(n, 256), 256, 0, h->stream>>>(G, SortRowsF64{h->pts, h->pitch}, n, h->s_bucket,
+                                                               h->s_count, h->err);
+    }
     CK_LAUNCH(h, "sort keys");
     r = exclusive_scan(h, h->s_count, h->s_start, nb1, 0);
     if (r) return r;
@@ -673,9 +674,23 @@ int do_sort_f64(mpm_handle* h) {
     CK(h, cudaMemcpyAsync(&kept, h->s_start + G.nb, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     if (kept > 0) {
-        dim3 grid(blocks_for(kept, 256), MPM_N_PTS_ARRAYS);
-        k_gather_rows<double><<<grid, 256, 0, h->stream>>>(h->pts, h->pitch, h->pts_alt, h->pitch, MPM_N_PTS_ARRAYS,
-                                                           h->s_perm, kept);
+        const unsigned gb = blocks_for(kept, 256);
+        if (mixed) {
+            // the 32-bit rows themselves, and the utility words, whose upper
+            // halves only the staging rows hold
+            k_gather_rows<float><<<dim3(gb, kGatherSplit), 256, 0, h->stream>>>(
+                static_cast<float*>(h->mx), h->pitch, static_cast<float*>(h->mx_alt), h->pitch, MPM_N_PTS_ARRAYS,
+                h->s_perm, kept);
+            std::swap(h->mx, h->mx_alt);
+            k_gather_rows<double><<<dim3(gb, 1), 256, 0, h->stream>>>(h->pts, h->pitch, h->pts_alt, h->pitch, 1,
+                                                                      h->s_perm, kept);
+            CK(h, cudaMemcpyAsync(h->pts, h->pts_alt, sizeof(double) * (size_t)kept, cudaMemcpyDeviceToDevice,
+                                  h->stream));
+        } else {
+            k_gather_rows<double><<<dim3(gb, kGatherSplit), 256, 0, h->stream>>>(
+                h->pts, h->pitch, h->pts_alt, h->pitch, MPM_N_PTS_ARRAYS, h->s_perm, kept);
+            std::swap(h->pts, h->pts_alt);
+        }
         CK_LAUNCH(h, "gather rows");
         k_gather_rows<unsigned><<<dim3(blocks_for(kept, 256), 1), 256, 0, h->stream>>>(h->ids, h->pitch, h->ids_alt,
                                                                                        h->pitch, 1, h->s_perm, kept);
@@ -686,8 +701,11 @@ int do_sort_f64(mpm_handle* h) {
                                                                                          h->pitch, 1, h->s_perm, kept);
             CK_LAUNCH(h, "gather p0");
             std::swap(h->p0, h->p0_alt);
+            if (mixed && h->p0f) {
+                k_narrow<<<blocks_for(kept, 256), 256, 0, h->stream>>>(h->p0, h->p0f, kept);
+                CK_LAUNCH(h, "p0 narrow");
+            }
         }
-        std::swap(h->pts, h->pts_alt);
         std::swap(h->ids, h->ids_alt);
     }
     h->n = (unsigned)kept;
@@ -2202,7 +2220,7 @@ extern "C" int mpm_sort_permutation_noalloc(const SimParams3D* prms, const doubl
         G.key_shift = prms->GridHaloSize * G.slab;
         G.nb = (int)nb;
         G.h_inv = prms->cellsize_inv;
-        k_sort_keys<<<blocks_for(n, 256), 256, 0, s>>>(G, soa, pitch, (int)n, bucket, count, err);
+        k_sort_keys<<<blocks_for(n, 256), 256, 0, s>>>(G, SortRowsF64{soa, pitch}, (int)n, bucket, count, err);
         CK_LAUNCH(nullptr, "noalloc sort keys");
         const int tiles = (nb1 + kScanTile - 1) / kScanTile;
         k_scan_tiles<<<tiles, kScanBlock, 0, s>>>(count, start, nb1, tiles > 1 ? sums : nullptr);
