@@ -105,13 +105,12 @@ __device__ __forceinline__ void p2g_alone(const DevParams& P, const P2GPoint& q,
 //
 // With the pairs alone the FP64 atomics bound the kernel (L2 and the path to
 // it at 78 %, 54.6 M RED sectors, 0.316 ms for 2 M points). The chains leave
-// 37 M sectors, and the latency of the shuffles and of the FP64 pipe becomes
-// what the time goes to: a stencil row's twelve sums are exchanged together
-// and the row ends in two predicates, at 124 registers without spills, 0.237
-// ms (64-thread blocks, 8 per SM; 10 at 96 registers: 0.242, 12 at 80: 0.245;
-// with a branch per quantity 0.279). Two points to a lane instead of the pair
-// merge (a list of slots per warp) took 0.30: no unit above 60 %, too few
-// warps for its latencies.
+// 37 M sectors, and the shuffles' LSU data pipe (78 %) is the busiest unit: a
+// stencil row's twelve sums are exchanged together and the row ends in two
+// predicates, at 124 registers without spills, 0.237 ms (64-thread blocks, 8
+// per SM; 10 at 96 registers: 0.242, 12 at 80: 0.245; with a branch per
+// quantity 0.279). Two points to a lane instead of the pair merge (a list of
+// slots per warp) took 0.30: no unit above 60 %, too few warps for its latencies.
 constexpr int kP2GBlock = 64;
 __global__ void __launch_bounds__(kP2GBlock, 8) k_p2g_pairs_f64(DevParams P, const double* __restrict__ pts,
                                                                   size_t pitch, int n, double* __restrict__ grid,
