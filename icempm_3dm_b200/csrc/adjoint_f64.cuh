@@ -288,10 +288,10 @@ struct AdjParams {
 // Together with the polar form of the map: the reverse sweep of 100,000 points
 // over 40 substeps, 3.5 % of them crushed, 20.3 -> 8.7 ms; this kernel 17 us.
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_adj_rm_vjp(DevParams P, AdjParams Q, const double* __restrict__ S0,
-                                                      const double* __restrict__ S1, size_t pitch,
-                                                      const int* __restrict__ list, const int* __restrict__ count,
-                                                      const double* __restrict__ p0arr, const double* __restrict__ A,
+__global__ void __launch_bounds__(BLOCK) k_adj_rm_vjp(DevParams P, AdjParams Q, const double* S0,
+                                                      const double* S1, size_t pitch,
+                                                      const int* list, const int* count,
+                                                      const double* __restrict__ p0arr, const double* A,
                                                       double* __restrict__ rmv, double* __restrict__ cgrad,
                                                       double* __restrict__ Egrad) {
     chain_wait();
@@ -363,10 +363,10 @@ inline unsigned rev_blocks(int n, int block, int lanes) {
 }
 
 template <int BLOCK, int LANES>
-__global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams Q, const double* __restrict__ S0,
-                                                       const double* __restrict__ S1, size_t pitch, int n,
-                                                       const double* __restrict__ g7,
-                                                       const double* __restrict__ rmv, double* __restrict__ A,
+__global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams Q, const double* S0,
+                                                       const double* S1, size_t pitch, int n,
+                                                       const double* g7,
+                                                       const double* rmv, double* __restrict__ A,
                                                        double* __restrict__ gadj) {
     chain_wait();
     const RevLane L = rev_lane<BLOCK, LANES>();
@@ -597,8 +597,8 @@ __global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, double* __r
 // ----------------------------------------------------------- reverse P2G
 
 template <int BLOCK, int LANES>
-__global__ void __launch_bounds__(BLOCK, 4) k_adj_p2g_rev(DevParams P, AdjParams Q, const double* __restrict__ S0,
-                                                       size_t pitch, int n, const double* __restrict__ gadj,
+__global__ void __launch_bounds__(BLOCK, 4) k_adj_p2g_rev(DevParams P, AdjParams Q, const double* S0,
+                                                       size_t pitch, int n, const double* gadj,
                                                        double* __restrict__ A, double* __restrict__ Egrad) {
     chain_wait();
     const RevLane L = rev_lane<BLOCK, LANES>();

@@ -51,6 +51,12 @@ struct DevParams {
 // serialisation attribute, so a kernel's blocks may be placed while the last
 // blocks of the one before it still run; they wait here until it has finished
 // and its writes are visible, and let the kernel after this one be placed.
+// So what the kernel before wrote is not read-only for this kernel's lifetime:
+// such data is read by plain loads after the wait, never through `const T*
+// __restrict__` parameters or __ldg, which promise that it is (the read-only
+// path may serve lines from before the wait, and such loads may be moved ahead
+// of it). Pointers that a kernel writes may be __restrict__: that speaks of
+// this kernel's own accesses only.
 __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -28,7 +28,7 @@ struct P2GPoint {
 };
 
 // Loads particle i and forms its P2G payload; false if disabled.
-__device__ __forceinline__ bool p2g_prepare(const DevParams& P, const double* __restrict__ pts, size_t pitch, int i,
+__device__ __forceinline__ bool p2g_prepare(const DevParams& P, const double* pts, size_t pitch, int i,
                                             P2GPoint& q, int* err) {
     const long long util = __double_as_longlong(pts[i]);
     if (util & kDisabled) return false;
@@ -112,7 +112,7 @@ __device__ __forceinline__ void p2g_alone(const DevParams& P, const P2GPoint& q,
 // quantity 0.279). Two points to a lane instead of the pair merge (a list of
 // slots per warp) took 0.30: no unit above 60 %, too few warps for its latencies.
 constexpr int kP2GBlock = 64;
-__global__ void __launch_bounds__(kP2GBlock, 8) k_p2g_pairs_f64(DevParams P, const double* __restrict__ pts,
+__global__ void __launch_bounds__(kP2GBlock, 8) k_p2g_pairs_f64(DevParams P, const double* pts,
                                                                   size_t pitch, int n, double* __restrict__ grid,
                                                                   int* err) {
     chain_wait();
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* grid,
 // Gathers v and C (APIC "Bp") of one particle from the updated grid
 // (mpm_kernels.cuh:278-305). Out-of-grid nodes contribute nothing.
 // grid: 4 arrays gstride apart, the node velocities in arrays 1-3 (array 0 is not read).
-__device__ __forceinline__ void g2p_gather(const DevParams& P, const double* __restrict__ grid, const double pos[3],
+__device__ __forceinline__ void g2p_gather(const DevParams& P, const double* grid, const double pos[3],
                                            double vel[3], double C[3][3], int* err) {
     int base[3];
     double fx[3];
@@ -390,7 +390,7 @@ __device__ __forceinline__ void g2p_gather(const DevParams& P, const double* __r
                 if (e && !node_inside(P, x, y, z)) continue;
                 const long long ni = ib + c;
                 const double w = wab * ww[c][2];
-                const double wn[3] = {w * __ldg(gx + ni), w * __ldg(gy + ni), w * __ldg(gz + ni)};
+                const double wn[3] = {w * gx[ni], w * gy[ni], w * gz[ni]};
 #pragma unroll
                 for (int r = 0; r < 3; r++) {
                     rb[r] += wn[r];
@@ -473,8 +473,8 @@ constexpr int kG2PF64Blocks = 14;
 // else in place on out (a second pointer costs this kernel 8 %: 72 registers).
 template <bool APART>
 __global__ void __launch_bounds__(kG2PBlock, kG2PF64Blocks) k_g2p_f64(
-    DevParams P, const double* __restrict__ src, double* __restrict__ out, size_t pitch, int n, const double* __restrict__ grid, int record_pq, int* err,
-    int* __restrict__ rm_list, int* __restrict__ rm_count) {
+    DevParams P, const double* src, double* __restrict__ out, size_t pitch, int n, const double* grid, int record_pq,
+    int* err, int* __restrict__ rm_list, int* __restrict__ rm_count) {
     chain_wait();
     const double* const pts = APART ? src : out;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(kG2PBlock, kG2PF64Blocks) k_g2p_f64(
 template <class K>
 __global__ void __launch_bounds__(128) k_return_map_f64(DevParams P, double* __restrict__ pts, size_t pitch,
                                                         const double* __restrict__ p0_arr,
-                                                        const int* __restrict__ rm_list, const int* __restrict__ count,
+                                                        const int* rm_list, const int* count,
                                                         int* __restrict__ next_count) {
     chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) *next_count = 0;

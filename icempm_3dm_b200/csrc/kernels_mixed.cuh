@@ -176,7 +176,7 @@ struct WxSlot {
 // Gathers v and C from the float4 velocity grid (mpm_kernels.cuh:278-305).
 // Node indices step from the base node by constant offsets (32-bit: the
 // handle checks that the grid has fewer than 2^31 nodes).
-__device__ __forceinline__ void g2p_gather_mixed(const DevParams& P, const float4* __restrict__ vel, const int base[3],
+__device__ __forceinline__ void g2p_gather_mixed(const DevParams& P, const float4* vel, const int base[3],
                                                  const float fx[3], float v[3], float C[3][3], bool check, WxSlot wx) {
     float ww[3][3];
     quad_weights<float>(fx, ww);
@@ -202,7 +202,7 @@ __device__ __forceinline__ void g2p_gather_mixed(const DevParams& P, const float
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 if (check && !node_inside(P, base[0] + a, base[1] + b, base[2] + c)) continue;
-                const float4 nd = __ldg(vel + ib + c);
+                const float4 nd = vel[ib + c];
                 const float w = wab * ww[c][2];
                 const float nv[3] = {nd.x, nd.y, nd.z};
                 const float dp[3] = {dpa, dpb, c - fx[2]};
@@ -227,7 +227,7 @@ __device__ __forceinline__ void g2p_gather_mixed(const DevParams& P, const float
 // whose stencil leaves the grid, take the global gather. Called by the whole
 // warp (the box, the loads and __syncwarp are warp-wide).
 template <int VCAP>
-__device__ __forceinline__ void g2p_gather_staged(const DevParams& P, const float4* __restrict__ vel,
+__device__ __forceinline__ void g2p_gather_staged(const DevParams& P, const float4* vel,
                                                   float4* __restrict__ vbox, bool part, bool active,
                                                   const int base[3], const float fx[3], float v[3], float C[3][3],
                                                   int lane, WxSlot wx) {
@@ -722,7 +722,7 @@ __device__ __forceinline__ void fused_payload(const DevParams& P, bool active, c
 constexpr int kVBoxNodes = 256;
 template <class Acc>
 __device__ __forceinline__ void fused_particle(const DevParams& P, const MixedState& s, int i, int n,
-                                               const float4* __restrict__ vel, Acc acc,
+                                               const float4* vel, Acc acc,
                                                int do_p2g, int record_pq, int store_vc, int* err,
                                                int* __restrict__ rm_list, int* __restrict__ rm_count,
                                                float4* __restrict__ vbox, WxSlot wx, int lane) {
@@ -776,7 +776,7 @@ __device__ __forceinline__ void fused_particle(const DevParams& P, const MixedSt
 constexpr int kFusedBlock = 64;
 template <class Acc>
 __global__ void __launch_bounds__(kFusedBlock, 1024 / kFusedBlock) k_g2p2g_mixed(
-    DevParams P, MixedState s, int n, const float4* __restrict__ vel, Acc acc, int do_p2g,
+    DevParams P, MixedState s, int n, const float4* vel, Acc acc, int do_p2g,
     int record_pq, int store_vc, int* err, int* __restrict__ rm_list, int* __restrict__ rm_count) {
     chain_wait();
     extern __shared__ __align__(128) float mixed_tile[];
@@ -793,8 +793,8 @@ __global__ void __launch_bounds__(kFusedBlock, 1024 / kFusedBlock) k_g2p2g_mixed
 // list holds *count indices; the kernel also clears next_count, the counter
 // the next fused launch appends to. Grid-stride over the list.
 template <class Acc>
-__global__ void __launch_bounds__(128) k_return_map_mixed(DevParams P, MixedState s, const int* __restrict__ rm_list,
-                                                          const int* __restrict__ count, int* __restrict__ next_count,
+__global__ void __launch_bounds__(128) k_return_map_mixed(DevParams P, MixedState s, const int* rm_list,
+                                                          const int* count, int* __restrict__ next_count,
                                                           Acc acc, int do_p2g, int* err) {
     chain_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) *next_count = 0;
