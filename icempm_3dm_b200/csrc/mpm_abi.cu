@@ -840,6 +840,12 @@ int mpm_update_constants(mpm_handle* h, const SimParams3D* prms) {
 int mpm_upload_soa(mpm_handle* h, const double* soa, unsigned pitch, unsigned n) {
     if (!h || (!soa && n) || pitch < n) return MPM_ERR_ARG;
     if (n > h->capacity) return MPM_ERR_CAPACITY;
+    // A point at exactly half a cell reads nodes that have no mass with a weight
+    // of exactly 0, and the node update writes only nodes with mass: no value (a
+    // NaN) that an earlier run left may be there. Once here, not at every empty
+    // node of every substep, which on a sparse grid doubles the update's writes.
+    if (h->gvel) CK(h, cudaMemsetAsync(h->gvel, 0, sizeof(float4) * (size_t)h->dp.nodes, h->stream));
+    if (h->gvel64) CK(h, cudaMemsetAsync(h->gvel64, 0, sizeof(double) * 4 * (size_t)h->dp.gstride, h->stream));
     if (n) {
         CK(h, cudaMemcpy2DAsync(h->pts, sizeof(double) * h->pitch, soa, sizeof(double) * pitch, sizeof(double) * n,
                                 MPM_N_PTS_ARRAYS, cudaMemcpyHostToDevice, h->stream));
