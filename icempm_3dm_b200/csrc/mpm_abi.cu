@@ -7,6 +7,7 @@
 // kernels_*.cuh / sort.cuh headers.
 
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
@@ -66,7 +67,7 @@ struct mpm_handle {
     double* p0 = nullptr;             // per-particle apex shift (optional)
     unsigned* ids = nullptr;          // upload index of each particle
     double* grid = nullptr;           // AoS {m, mv} per node
-    double* gvel64 = nullptr;         // FP64 node velocities between the substeps of a call (arrays 1-3 of 4 x gstride)
+    double* gvel64 = nullptr;         // FP64 node velocities between the substeps of a call (3 x gstride; optional)
     double* sensor = nullptr;         // 3 * subdiv * Gz
     double* force_steps = nullptr;    // 3 per substep of the running mpm_step
     int force_steps_cap = 0;
@@ -129,6 +130,7 @@ struct mpm_handle {
     std::vector<int*> fr_scan_levels;
     bool fr_ready = false;            // a full frame has built the visual state
     cudaError_t last_cuda = cudaSuccess;
+    int fail_alloc = 0;               // test hook: the fail_alloc-th allocation from now fails
 
     // x-slab partition (mpm_set_partition); whole grid when part_gxp == 0
     int part_id = 0, part_x0 = 0, part_gxp = 0;
@@ -204,6 +206,8 @@ cudaError_t pool_for(int device, cudaMemPool_t* out) {
     return cudaSuccess;
 }
 
+bool release_optional(mpm_handle* h);
+
 template <class T>
 cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes) {
     *ptr = nullptr;
@@ -211,13 +215,23 @@ cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes) {
     cudaError_t e = pool_for(h->device, &pool);
     if (e != cudaSuccess) return e;
     void* p = nullptr;
-    e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
-    if (e == cudaErrorMemoryAllocation) {   // once more without what the pool holds for nobody
-        cudaGetLastError();
+    if (h->fail_alloc > 0 && --h->fail_alloc == 0) {
+        e = cudaErrorMemoryAllocation;
+    } else {
+        e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
+        if (e == cudaErrorMemoryAllocation) {   // once more without what the pool holds for nobody
+            cudaMemPoolTrimTo(pool, 0);
+            e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
+        }
+    }
+    if (e == cudaErrorMemoryAllocation && release_optional(h)) {   // and without what the handle can do without
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
     }
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // reported here: not again by the next launch
+        return e;
+    }
     // a caller's stream may use the memory at once
     if (h->stream != h->own_stream && (e = cudaStreamSynchronize(h->own_stream)) != cudaSuccess) return e;
     *ptr = static_cast<T*>(p);
@@ -226,6 +240,17 @@ cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes) {
 
 // The work that used the memory has completed (the callers synchronise first).
 cudaError_t dev_free(mpm_handle* h, void* p) { return p ? cudaFreeAsync(p, h->own_stream) : cudaSuccess; }
+
+// Gives up the buffers that only save time; false if there was none. They are
+// never taken while a call launches its kernels, but an allocation inside a call
+// (the first sort of a run) may find their last kernel still running.
+bool release_optional(mpm_handle* h) {
+    if (!h->gvel64) return false;
+    cudaStreamSynchronize(h->stream);
+    dev_free(h, h->gvel64);
+    h->gvel64 = nullptr;
+    return cudaStreamSynchronize(h->own_stream) == cudaSuccess;
+}
 
 void pool_enter(int device) {
     PoolTable& t = pools();
@@ -560,28 +585,39 @@ int reset_grid(mpm_handle* h) {
     return MPM_OK;
 }
 
-// P2G, node update and G2P of substep s of a run of nsteps (FP64 modes). Between
-// the substeps the update itself clears the sums, so only the first one clears
-// the grid; the last leaves m and v in it, as the phase calls do.
+// The grid that g2p_gather takes for node velocities in 3 arrays of their own.
+const double* gather_base(const mpm_handle* h, const double* vel) {
+    return reinterpret_cast<const double*>(reinterpret_cast<uintptr_t>(vel) - sizeof(double) * (size_t)h->dp.gstride);
+}
+
+// Before a run of nsteps substeps (FP64 modes): the velocities' buffer. Where
+// there is no memory for it (24 bytes a node) the substeps do without.
+int ensure_gvel64(mpm_handle* h, int nsteps) {
+    if (h->gvel64 || nsteps < 2) return MPM_OK;
+    const size_t bytes = sizeof(double) * 3 * (size_t)h->dp.gstride;
+    const cudaError_t e = dev_alloc(h, &h->gvel64, bytes);
+    if (e == cudaErrorMemoryAllocation) return MPM_OK;
+    CK(h, e);
+    CK(h, cudaMemsetAsync(h->gvel64, 0, bytes, h->stream));
+    return MPM_OK;
+}
+
+// P2G, node update and G2P of substep s of a run of nsteps (FP64 modes). With a
+// buffer for the velocities the update itself clears the sums between the
+// substeps, so only the first one clears the grid; the last leaves m and v in it,
+// as the phase calls do. Without the buffer every substep works in place.
 int fp64_grid_step(mpm_handle* h, int s, int nsteps, double* force3) {
     const SimParams3D& p = h->prms;
     int r;
-    const bool last = s == nsteps - 1;
-    if (!last && !h->gvel64) {
-        const size_t bytes = sizeof(double) * 4 * (size_t)h->dp.gstride;
-        CK(h, dev_alloc(h, &h->gvel64, bytes));
-        CK(h, cudaMemsetAsync(h->gvel64, 0, bytes, h->stream));
-    }
-    if (s == 0 && (r = reset_grid(h))) return r;
+    if ((s == 0 || !h->gvel64) && (r = reset_grid(h))) return r;
     if ((r = launch_p2g(h))) return r;
     const int record = (p.SimulationStep % p.UpdateEveryNthStep) == 0;
-    if (last) {
+    if (s == nsteps - 1 || !h->gvel64) {
         if ((r = launch_update(h, p.indenter_x, p.indenter_y, force3))) return r;
         return launch_g2p(h, record);
     }
-    if ((r = launch_update(h, p.indenter_x, p.indenter_y, force3, kVelClear, h->grid,
-                           h->gvel64 + h->dp.gstride))) return r;
-    return launch_g2p(h, record, h->gvel64);
+    if ((r = launch_update(h, p.indenter_x, p.indenter_y, force3, kVelClear, h->grid, h->gvel64))) return r;
+    return launch_g2p(h, record, gather_base(h, h->gvel64));
 }
 
 int read_error(mpm_handle* h, int* code) {
@@ -845,7 +881,7 @@ int mpm_upload_soa(mpm_handle* h, const double* soa, unsigned pitch, unsigned n)
     // NaN) that an earlier run left may be there. Once here, not at every empty
     // node of every substep, which on a sparse grid doubles the update's writes.
     if (h->gvel) CK(h, cudaMemsetAsync(h->gvel, 0, sizeof(float4) * (size_t)h->dp.nodes, h->stream));
-    if (h->gvel64) CK(h, cudaMemsetAsync(h->gvel64, 0, sizeof(double) * 4 * (size_t)h->dp.gstride, h->stream));
+    if (h->gvel64) CK(h, cudaMemsetAsync(h->gvel64, 0, sizeof(double) * 3 * (size_t)h->dp.gstride, h->stream));
     if (n) {
         CK(h, cudaMemcpy2DAsync(h->pts, sizeof(double) * h->pitch, soa, sizeof(double) * pitch, sizeof(double) * n,
                                 MPM_N_PTS_ARRAYS, cudaMemcpyHostToDevice, h->stream));
@@ -1134,6 +1170,8 @@ int mpm_step(mpm_handle* h, int nsteps, double* force_hist) {
         if ((r = launch_p2g(h))) return r;
         h->p2g_ready = true;
     }
+    if (!is_mixed(h))
+        if (const int r = ensure_gvel64(h, nsteps)) return r;
     for (int s = 0; s < nsteps; s++) {
         p.SimulationTime += p.InitialTimeStep;
         p.indenter_x = p.indenter_x_initial + p.SimulationTime * p.IndVelocity;
@@ -2029,6 +2067,13 @@ int mpm_testing_svd3x3(int mode, const double* A, int count, double* U, double* 
 
 size_t mpm_testing_sizeof_params(void) { return sizeof(SimParams3D); }
 
+int mpm_testing_fail_alloc(mpm_handle* h, int k) {
+    if (!h) return -1;
+    const int left = h->fail_alloc;
+    h->fail_alloc = k;
+    return left;
+}
+
 int mpm_testing_step_timed(mpm_handle* h, int nsteps, float* ms) {
     if (!h || nsteps <= 0 || !ms) return MPM_ERR_ARG;
     if (!h->uploaded) return MPM_ERR_STATE;
@@ -2402,6 +2447,7 @@ extern "C" int mpm_adjoint_forward(mpm_handle* h, int nsteps, int ckpt_every, do
         CK(h, dev_alloc(h, &h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
         h->force_steps_cap = nsteps;
     }
+    if ((r = ensure_gvel64(h, nsteps))) return r;
     CK(h, cudaMemsetAsync(h->force_steps, 0, sizeof(double) * 3 * (size_t)nsteps, h->stream));
     for (int s = 0; s < nsteps; s++) {
         if (s % ckpt_every == 0) {

@@ -39,6 +39,12 @@ int mpm_testing_active_nodes(mpm_handle* h, long long* count);
 /* sizeof(SimParams3D) as compiled into the library (layout check). */
 size_t mpm_testing_sizeof_params(void);
 
+/* Makes the k-th allocation of device memory that the handle asks for from
+ * now on find none left (0: no failure): it fails, unless the handle holds a
+ * buffer that it can do without and give up for it. Returns what was left of
+ * an earlier count: 0 if its turn has come. */
+int mpm_testing_fail_alloc(mpm_handle* h, int k);
+
 #ifdef __cplusplus
 }
 #endif
