@@ -365,7 +365,7 @@ inline unsigned rev_blocks(int n, int block, int lanes) {
 template <int BLOCK, int LANES>
 __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams Q, const double* S0,
                                                        const double* S1, size_t pitch, int n,
-                                                       const double* g7,
+                                                       const double* nodes,
                                                        const double* rmv, double* __restrict__ A,
                                                        double* __restrict__ gadj) {
     chain_wait();
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams
                     const double wt = wa * w[b][1] * w[c][2];
                     const double gw[3] = {dwa * w[b][1] * w[c][2], wa * dwh[b][1] * w[c][2],
                                           wa * w[b][1] * dwh[c][2]};
-                    const double nv[3] = {g7[4 * P.gstride + ni], g7[5 * P.gstride + ni], g7[6 * P.gstride + ni]};
+                    const double nv[3] = {nodes[ni], nodes[P.gstride + ni], nodes[2 * P.gstride + ni]};
                     const double dd[3] = {(a - fx[0]) * h, (b - fx[1]) * h, (c - fx[2]) * h};
                     double gsc = 0;
 #pragma unroll
@@ -508,17 +508,17 @@ __global__ void __launch_bounds__(BLOCK, 3) k_adj_g2p_rev(DevParams P, AdjParams
 // ---------------------------------------------------------- reverse node
 
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, double* __restrict__ g7,
+__global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, double* __restrict__ sums,
                                                         double* __restrict__ gadj, double ind_x, double ind_y,
                                                         double fb0, double fb1, double fb2) {
     chain_wait();
     const long long idx = (long long)blockIdx.x * BLOCK + threadIdx.x;
     if (idx >= P.nodes) return;
     const long long gs = P.gstride;
-    const double mass = g7[idx];
+    const double mass = sums[idx];
     double mb = 0, Pb[3] = {0, 0, 0};
     if (mass != 0) {
-        const double Pm[3] = {g7[gs + idx], g7[2 * gs + idx], g7[3 * gs + idx]};
+        const double Pm[3] = {sums[gs + idx], sums[2 * gs + idx], sums[3 * gs + idx]};
         double v1[3] = {Pm[0] / mass, Pm[1] / mass - P.dt_gravity, Pm[2] / mass};
         const int idx_z = (int)(idx % P.Gz), idx_y = (int)((idx / P.Gz) % P.Gy), idx_x = (int)(idx / P.slab);
         const int gx = idx_x - P.halo, gy = idx_y, gz = idx_z;
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_node_rev(DevParams P, double* __r
         }
         // both are summed into again: the sums by a later segment's P2G, the
         // velocity adjoints by the next substep's reverse G2P
-        for (int k = 0; k < 4; k++) g7[k * gs + idx] = 0.0;
+        for (int k = 0; k < 4; k++) sums[k * gs + idx] = 0.0;
         for (int k = 0; k < 3; k++) gadj[k * gs + idx] = 0.0;
     }
     gadj[3 * gs + idx] = mb;

@@ -213,8 +213,10 @@ __global__ void __launch_bounds__(kP2GBlock, 8) k_p2g_pairs_f64(DevParams P, con
 // force3 receives the block-reduced force of this substep (3 doubles).
 // One node with mass of partition_kernel_update_nodes: v (the node's momentum
 // on entry) becomes its velocity; the contact force goes to f and the sensor.
-__device__ __forceinline__ void update_node_f64(const DevParams& P, double* vel, long long idx, double mass, double v[3], double ind_x, double ind_y,
-                                                double* __restrict__ sensor, double f[3]) {
+template <bool FORCE>
+__device__ __forceinline__ void update_node_f64(const DevParams& P, double* vel, long long idx, double mass,
+                                                double v[3], double ind_x, double ind_y, double* __restrict__ sensor,
+                                                double f[3]) {
     int idx_z, idx_y;
     const long long col = div_by64(idx, P.Gz, P.inv_gz, idx_z);
     const int idx_x = (int)div_by64(col, P.Gy, P.inv_gy, idx_y);
@@ -243,7 +245,7 @@ __device__ __forceinline__ void update_node_f64(const DevParams& P, double* vel,
                 v[2] = vt[2];
                 // a node in the overlap of two partitions is updated
                 // by both; its force is counted by its owner only
-                if (gx >= P.own_lo && gx < P.own_hi) {
+                if (FORCE && gx >= P.own_lo && gx < P.own_hi) {
                     double fn[3];
 #pragma unroll
                     for (int k = 0; k < 3; k++) { fn[k] = (prev[k] - v[k]) * mass / P.dt; f[k] += fn[k]; }
@@ -293,7 +295,8 @@ __device__ __forceinline__ void update_node_f64(const DevParams& P, double* vel,
 //                (no clearing pass of its own between the substeps)
 //   kVelRecord   to another buffer, zero where there is no mass; the sums stay
 //                (the reverse sweep reads both)
-enum { kVelInPlace = 0, kVelClear = 1, kVelRecord = 2 };
+//   kVelOnly     as kVelRecord, without the force: the velocities once more
+enum { kVelInPlace = 0, kVelClear = 1, kVelRecord = 2, kVelOnly = 3 };
 constexpr int kUpdateF64NodesPerThread = 2;
 template <int BLOCK, int MODE>
 __global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* grid, double* vel, double ind_x, double ind_y,
@@ -321,12 +324,13 @@ __global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* grid,
             for (int k = 0; k < 4; k++) grid[k * P.gstride + idx] = 0.0;
         }
         if (m[j] != 0) {
-            update_node_f64(P, vel, idx, m[j], v[j], ind_x, ind_y, sensor, f);
-        } else if (MODE == kVelRecord && idx < P.node_hi) {
+            update_node_f64<MODE != kVelOnly>(P, vel, idx, m[j], v[j], ind_x, ind_y, sensor, f);
+        } else if ((MODE == kVelRecord || MODE == kVelOnly) && idx < P.node_hi) {
 #pragma unroll
             for (int k = 0; k < 3; k++) vel[k * P.gstride + idx] = 0.0;
         }
     }
+    if (MODE == kVelOnly) return;
     // block reduction of the substep force (only blocks that touch the
     // indenter contribute non-zero values)
     __shared__ double red[3][BLOCK / 32];

@@ -114,12 +114,12 @@ struct mpm_handle {
     bool adj_ready = false;
     double* adj_force = nullptr;      // force history of a mixed adjoint forward (3 per substep)
     int adj_force_cap = 0;
-    std::vector<double*> adj_gcache;  // grid of each substep of the segment being reversed: m, P, v (7 x gstride)
+    std::vector<double*> adj_gcache;  // grid of each substep of the segment being reversed: m, P (4 x gstride)
+    std::vector<double*> adj_vel;     // and its node velocities (3 x gstride); one for all where memory is short
+    bool adj_lean = false;            // memory was too short for more than one of adj_vel
     double* adj_rmv = nullptr;        // return-map VJP of the crushed points (10 x pitch)
-    int* adj_rml = nullptr;           // crushed points of each substep of the segment (pitch per substep)
-    int* adj_rmc = nullptr;           // and their counts
-    int adj_rm_cap = 0;               // substeps the two hold
-
+    int* adj_rmc = nullptr;           // counts of the points that each substep of the segment crushed
+    int adj_rmc_cap = 0;              // substeps that it holds
 
     // animation-frame records (mpm_frame_records), allocated on first use
     float* fr_f = nullptr;            // visual state: pos 3, vel 3, Jp_inv rows x pitch
@@ -208,8 +208,9 @@ cudaError_t pool_for(int device, cudaMemPool_t* out) {
 
 bool release_optional(mpm_handle* h);
 
+// optional: a buffer that only saves time, for which no other one is given up.
 template <class T>
-cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes) {
+cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes, bool optional = false) {
     *ptr = nullptr;
     cudaMemPool_t pool;
     cudaError_t e = pool_for(h->device, &pool);
@@ -224,7 +225,7 @@ cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes) {
             e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
         }
     }
-    if (e == cudaErrorMemoryAllocation && release_optional(h)) {   // and without what the handle can do without
+    if (e == cudaErrorMemoryAllocation && !optional && release_optional(h)) {   // and without what the handle can do without
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
     }
@@ -245,10 +246,11 @@ cudaError_t dev_free(mpm_handle* h, void* p) { return p ? cudaFreeAsync(p, h->ow
 // never taken while a call launches its kernels, but an allocation inside a call
 // (the first sort of a run) may find their last kernel still running.
 bool release_optional(mpm_handle* h) {
-    if (!h->gvel64) return false;
+    if (!h->gvel64 && h->adj_vel.size() < 2) return false;
     cudaStreamSynchronize(h->stream);
     dev_free(h, h->gvel64);
     h->gvel64 = nullptr;
+    for (; h->adj_vel.size() > 1; h->adj_vel.pop_back()) dev_free(h, h->adj_vel.back());
     return cudaStreamSynchronize(h->own_stream) == cudaSuccess;
 }
 
@@ -367,7 +369,9 @@ void free_all(mpm_handle* h) {
     dev_free(h, h->adj_force);
     for (double* c : h->adj_gcache) dev_free(h, c);
     h->adj_gcache.clear();
-    dev_free(h, h->adj_rmv); dev_free(h, h->adj_rml); dev_free(h, h->adj_rmc);
+    for (double* c : h->adj_vel) dev_free(h, c);
+    h->adj_vel.clear();
+    dev_free(h, h->adj_rmv); dev_free(h, h->adj_rmc);
     for (int* p : h->scan_levels) dev_free(h, p);
     h->scan_levels.clear();
     dev_free(h, h->fr_f); dev_free(h, h->fr_status); dev_free(h, h->fr_last); dev_free(h, h->fr_i); dev_free(h, h->fr_rec);
@@ -486,8 +490,10 @@ int launch_update(mpm_handle* h, double ind_x, double ind_y, double* force3, int
               ind_y, h->sensor, force3);
     else if (mode == kVelClear)
         chain(k_update_f64<256, kVelClear>, nb, 256, 0, h->stream, h->dp, acc, vel, ind_x, ind_y, h->sensor, force3);
-    else
+    else if (mode == kVelRecord)
         chain(k_update_f64<256, kVelRecord>, nb, 256, 0, h->stream, h->dp, acc, vel, ind_x, ind_y, h->sensor, force3);
+    else
+        chain(k_update_f64<256, kVelOnly>, nb, 256, 0, h->stream, h->dp, acc, vel, ind_x, ind_y, h->sensor, force3);
     CK_LAUNCH(h, "update kernel");
     return MPM_OK;
 }
@@ -595,7 +601,7 @@ const double* gather_base(const mpm_handle* h, const double* vel) {
 int ensure_gvel64(mpm_handle* h, int nsteps) {
     if (h->gvel64 || nsteps < 2) return MPM_OK;
     const size_t bytes = sizeof(double) * 3 * (size_t)h->dp.gstride;
-    const cudaError_t e = dev_alloc(h, &h->gvel64, bytes);
+    const cudaError_t e = dev_alloc(h, &h->gvel64, bytes, true);
     if (e == cudaErrorMemoryAllocation) return MPM_OK;
     CK(h, e);
     CK(h, cudaMemsetAsync(h->gvel64, 0, bytes, h->stream));
@@ -2307,25 +2313,27 @@ void advance_indenter(mpm_handle* h) {
     p.indenter_x = p.indenter_x_initial + p.SimulationTime * p.IndVelocity;
 }
 
-// One recomputed FP64 substep of Model3D::Step, from the particle rows src to
-// the rows out: the sums and velocities stay in the 7 arrays of g7 (m, P, v;
-// the sums zero on entry), the points that it crushed in rm_list and rm_count
-// (zeroed).
-int fp64_recompute(mpm_handle* h, const double* src, double* out, double* g7, int* rm_list, int* rm_count) {
+// The points that substep m of the segment crushed: their list has its place in
+// the P row of the state after it, which no recomputed substep records.
+int* crushed_list(mpm_handle* h, int m) { return reinterpret_cast<int*>(h->seg[m] + MPM_IDX_P * h->pitch); }
+
+// One recomputed FP64 substep of Model3D::Step, number m of its segment, from the
+// particle rows src to seg[m]: the sums stay in adj_gcache[m] (zero on entry), the
+// velocities in vel, the points that it crushed in their list.
+int fp64_recompute(mpm_handle* h, int m, const double* src, double* vel) {
     SimParams3D& p = h->prms;
     advance_indenter(h);
-    double* const vgrid = g7 + 3 * h->dp.gstride;   // its arrays 1-3: arrays 4-6 of g7
     int r;
-    if ((r = launch_p2g(h, src, g7))) return r;
-    if ((r = launch_update(h, p.indenter_x, p.indenter_y, h->force_phase, kVelRecord, g7,
-                           vgrid + h->dp.gstride))) return r;
-    if ((r = launch_g2p(h, 0, vgrid, src, out, rm_list, rm_count))) return r;
+    if ((r = launch_p2g(h, src, h->adj_gcache[m]))) return r;
+    if ((r = launch_update(h, p.indenter_x, p.indenter_y, h->force_phase, kVelRecord, h->adj_gcache[m], vel))) return r;
+    if ((r = launch_g2p(h, 0, gather_base(h, vel), src, h->seg[m], crushed_list(h, m), h->adj_rmc + m))) return r;
     p.SimulationStep += 1;
     return MPM_OK;
 }
 
 int ensure_adjoint_buffers(mpm_handle* h, int nsteps, int every) {
     const int nck = (nsteps + every - 1) / every;
+    const size_t gs = (size_t)h->dp.gstride;
     while ((int)h->ckpt.size() < nck) {
         double* b = nullptr;
         CK(h, dev_alloc(h, &b, state_bytes(h)));
@@ -2338,20 +2346,17 @@ int ensure_adjoint_buffers(mpm_handle* h, int nsteps, int every) {
     }
     while ((int)h->adj_gcache.size() < every) {
         double* b = nullptr;
-        CK(h, dev_alloc(h, &b, sizeof(double) * 7 * (size_t)h->dp.gstride));
+        CK(h, dev_alloc(h, &b, sizeof(double) * 4 * gs));
         h->adj_gcache.push_back(b);
-        CK(h, cudaMemsetAsync(b, 0, sizeof(double) * 7 * (size_t)h->dp.gstride, h->stream));
     }
     h->ckpt_prms.resize(nck);
-    if (every > h->adj_rm_cap) {
+    if (every > h->adj_rmc_cap) {
         CK(h, cudaStreamSynchronize(h->stream));
-        dev_free(h, h->adj_rml);
         dev_free(h, h->adj_rmc);
-        h->adj_rml = h->adj_rmc = nullptr;
-        h->adj_rm_cap = 0;
-        CK(h, dev_alloc(h, &h->adj_rml, sizeof(int) * h->pitch * (size_t)every));
+        h->adj_rmc = nullptr;
+        h->adj_rmc_cap = 0;
         CK(h, dev_alloc(h, &h->adj_rmc, sizeof(int) * (size_t)every));
-        h->adj_rm_cap = every;
+        h->adj_rmc_cap = every;
     }
     if (!h->adj_A) {
         CK(h, dev_alloc(h, &h->adj_A, sizeof(double) * ADJ_ROWS * h->pitch));
@@ -2359,6 +2364,25 @@ int ensure_adjoint_buffers(mpm_handle* h, int nsteps, int every) {
         CK(h, dev_alloc(h, &h->adj_Egrad, sizeof(double)));
         CK(h, dev_alloc(h, &h->adj_gb7, sizeof(double) * 7 * (size_t)h->dp.gstride));
         CK(h, dev_alloc(h, &h->adj_rmv, sizeof(double) * 10 * h->pitch));
+    }
+    // Last, since all but the first can be done without: the velocities of the
+    // segment's substeps. With one buffer for all, the reverse sweep does the node
+    // update of each substep again: 40 substeps of 20,000 points 3.14 -> 3.25 ms,
+    // 100,000 5.97 -> 6.07, 500,000 21.6 -> 21.7.
+    while ((int)h->adj_vel.size() < (h->adj_lean ? 1 : every)) {
+        double* b = nullptr;
+        const bool first = h->adj_vel.empty();
+        const cudaError_t e = dev_alloc(h, &b, sizeof(double) * 3 * gs, !first);
+        if (e == cudaErrorMemoryAllocation && !first) {
+            h->adj_lean = true;
+            release_optional(h);
+            break;
+        }
+        CK(h, e);
+        h->adj_vel.push_back(b);
+        // the node update writes every node of the window, so of the whole grid
+        if (h->dp.node_lo != 0 || h->dp.node_hi != h->dp.nodes)
+            CK(h, cudaMemsetAsync(b, 0, sizeof(double) * 3 * gs, h->stream));
     }
     return MPM_OK;
 }
@@ -2478,6 +2502,7 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
     const AdjParams q = adj_params(h);
     const size_t gs = (size_t)dp.gstride;
     const bool split = n <= kRevSplitPerSM * h->num_sms;
+    const bool lean = (int)h->adj_vel.size() < std::min(k, N);   // one velocity buffer for the segment's substeps
     CK(h, cudaMemsetAsync(h->adj_A, 0, sizeof(double) * ADJ_ROWS * h->pitch, h->stream));
     CK(h, cudaMemsetAsync(h->adj_cgrad, 0, sizeof(double) * h->pitch, h->stream));
     CK(h, cudaMemsetAsync(h->adj_Egrad, 0, sizeof(double), h->stream));
@@ -2497,8 +2522,7 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
         h->prms = h->ckpt_prms[j];
         CK(h, cudaMemsetAsync(h->adj_rmc, 0, sizeof(int) * (size_t)(s1 - s0), h->stream));
         for (int m = 0; m < s1 - s0 && !r; m++) {
-            r = fp64_recompute(h, S[m], h->seg[m], h->adj_gcache[m], h->adj_rml + h->pitch * (size_t)m,
-                               h->adj_rmc + m);
+            r = fp64_recompute(h, m, S[m], h->adj_vel[lean ? 0 : m]);
             S[m + 1] = h->seg[m];
             sp[m] = h->prms;   // holds this substep's indenter position
         }
@@ -2507,14 +2531,16 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
         for (int m = s1 - s0 - 1; m >= 0; m--) {
             const double* dl = dL_dforce + 3 * (size_t)(s0 + m);
             const double ix = sp[m].indenter_x, iy = sp[m].indenter_y;
-            double* const g7 = h->adj_gcache[m];
+            double* const sums = h->adj_gcache[m];
+            double* const vel = h->adj_vel[lean ? 0 : m];
+            if (lean && m < s1 - s0 - 1 && (r = launch_update(h, ix, iy, h->force_phase, kVelOnly, sums, vel))) break;
             chain(k_adj_rm_vjp<128>, h->num_sms * 4, 128, 0, h->stream, dp, q, S[m], S[m + 1], h->pitch,
-                  h->adj_rml + h->pitch * (size_t)m, h->adj_rmc + m, h->p0, h->adj_A, h->adj_rmv, h->adj_cgrad,
+                  crushed_list(h, m), h->adj_rmc + m, h->p0, h->adj_A, h->adj_rmv, h->adj_cgrad,
                   h->adj_Egrad);
             const unsigned nb = rev_blocks(n, 128, split ? 3 : 1);
             chain(split ? k_adj_g2p_rev<128, 3> : k_adj_g2p_rev<128, 1>, nb, 128, 0, h->stream, dp, q, S[m], S[m + 1],
-                  h->pitch, n, g7, h->adj_rmv, h->adj_A, h->adj_gb7);
-            chain(k_adj_node_rev<256>, blocks_for(dp.nodes, 256), 256, 0, h->stream, dp, g7, h->adj_gb7, ix, iy, dl[0],
+                  h->pitch, n, vel, h->adj_rmv, h->adj_A, h->adj_gb7);
+            chain(k_adj_node_rev<256>, blocks_for(dp.nodes, 256), 256, 0, h->stream, dp, sums, h->adj_gb7, ix, iy, dl[0],
                   dl[1], dl[2]);
             chain(split ? k_adj_p2g_rev<128, 3> : k_adj_p2g_rev<128, 1>, nb, 128, 0, h->stream, dp, q, S[m], h->pitch,
                   n, h->adj_gb7, h->adj_A, h->adj_Egrad);
