@@ -84,7 +84,7 @@ struct mpm_handle {
     int* s_start = nullptr;
     unsigned* s_perm = nullptr;
     std::vector<int*> scan_levels;    // per-level tile sums and their scans
-    std::vector<int> scan_sizes;
+    bool sort_ready = false;          // all of it is there
     int sort_interval = 0;
     int steps_since_sort = 0;
 
@@ -241,6 +241,42 @@ cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes, bool optional = fals
 
 // The work that used the memory has completed (the callers synchronise first).
 cudaError_t dev_free(mpm_handle* h, void* p) { return p ? cudaFreeAsync(p, h->own_stream) : cudaSuccess; }
+
+// A buffer made on first use, unless an earlier call has made it: where a group of
+// them stopped half way for want of memory, the next call makes the rest.
+template <class T>
+cudaError_t dev_ensure(mpm_handle* h, T** ptr, size_t bytes) {
+    return *ptr ? cudaSuccess : dev_alloc(h, ptr, bytes);
+}
+
+// A buffer of count entries that has to grow: the old one goes when the new one is there.
+template <class T>
+cudaError_t dev_grow(mpm_handle* h, T** ptr, int* have, int count, size_t entry) {
+    if (*ptr && count <= *have) return cudaSuccess;
+    T* p = nullptr;
+    cudaError_t e = dev_alloc(h, &p, entry * (size_t)count);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess || (e = dev_free(h, *ptr)) != cudaSuccess) {
+        dev_free(h, p);
+        return e;
+    }
+    *ptr = p;
+    *have = count;
+    return cudaSuccess;
+}
+
+// Tile sums and their scans, level by level, for exclusive_scan over m entries.
+cudaError_t ensure_scan_levels(mpm_handle* h, std::vector<int*>& lv, long long m, int tile) {
+    for (size_t k = 0; m > tile; k += 2) {
+        m = (m + tile - 1) / tile;
+        if (lv.size() < k + 2) lv.resize(k + 2, nullptr);
+        for (size_t j = k; j < k + 2; j++) {
+            const cudaError_t e = dev_ensure(h, &lv[j], sizeof(int) * (size_t)m);
+            if (e != cudaSuccess) return e;
+        }
+    }
+    return cudaSuccess;
+}
 
 // Gives up the buffers that only save time; false if there was none. They are
 // never taken while a call launches its kernels, but an allocation inside a call
@@ -635,29 +671,21 @@ int read_error(mpm_handle* h, int* code) {
 // ------------------------------------------------------------------ sort
 
 int ensure_sort_scratch(mpm_handle* h) {
-    if (h->s_bucket) return MPM_OK;
+    if (h->p0) CK(h, dev_ensure(h, &h->p0_alt, sizeof(double) * h->pitch));
+    if (h->sort_ready) return MPM_OK;
     const SimParams3D& p = h->prms;
     const long long nb = (long long)(p.GridXTotal + 2 * p.GridHaloSize + 1) * p.GridY * p.GridZ;
     if (nb + 1 > 0x7fffffffLL) return MPM_ERR_ARG;
     const bool mixed = is_mixed(h);
-    CK(h, dev_alloc(h, &h->pts_alt, sizeof(double) * (mixed ? 1 : MPM_N_PTS_ARRAYS) * h->pitch));
-    if (mixed) CK(h, dev_alloc(h, &h->mx_alt, sizeof(float) * MPM_N_PTS_ARRAYS * h->pitch));
-    CK(h, dev_alloc(h, &h->ids_alt, sizeof(unsigned) * h->pitch));
-    CK(h, dev_alloc(h, &h->s_bucket, sizeof(int) * h->pitch));
-    CK(h, dev_alloc(h, &h->s_perm, sizeof(unsigned) * h->pitch));
-    CK(h, dev_alloc(h, &h->s_count, sizeof(int) * (nb + 1)));
-    CK(h, dev_alloc(h, &h->s_start, sizeof(int) * (nb + 1)));
-    long long m = nb + 1;
-    while (m > kScanTile) {
-        m = (m + kScanTile - 1) / kScanTile;
-        int* sums = nullptr;
-        int* scanned = nullptr;
-        CK(h, dev_alloc(h, &sums, sizeof(int) * m));
-        CK(h, dev_alloc(h, &scanned, sizeof(int) * m));
-        h->scan_levels.push_back(sums);
-        h->scan_levels.push_back(scanned);
-        h->scan_sizes.push_back((int)m);
-    }
+    CK(h, dev_ensure(h, &h->pts_alt, sizeof(double) * (mixed ? 1 : MPM_N_PTS_ARRAYS) * h->pitch));
+    if (mixed) CK(h, dev_ensure(h, &h->mx_alt, sizeof(float) * MPM_N_PTS_ARRAYS * h->pitch));
+    CK(h, dev_ensure(h, &h->ids_alt, sizeof(unsigned) * h->pitch));
+    CK(h, dev_ensure(h, &h->s_bucket, sizeof(int) * h->pitch));
+    CK(h, dev_ensure(h, &h->s_perm, sizeof(unsigned) * h->pitch));
+    CK(h, dev_ensure(h, &h->s_count, sizeof(int) * (nb + 1)));
+    CK(h, dev_ensure(h, &h->s_start, sizeof(int) * (nb + 1)));
+    CK(h, ensure_scan_levels(h, h->scan_levels, nb + 1, kScanTile));
+    h->sort_ready = true;
     return MPM_OK;
 }
 
@@ -738,7 +766,6 @@ int do_sort(mpm_handle* h) {
                                                                                        h->pitch, 1, h->s_perm, kept);
         CK_LAUNCH(h, "gather ids");
         if (h->p0) {
-            if (!h->p0_alt) CK(h, dev_alloc(h, &h->p0_alt, sizeof(double) * h->pitch));
             k_gather_rows<double><<<dim3(blocks_for(kept, 256), 1), 256, 0, h->stream>>>(h->p0, h->pitch, h->p0_alt,
                                                                                          h->pitch, 1, h->s_perm, kept);
             CK_LAUNCH(h, "gather p0");
@@ -920,8 +947,15 @@ int mpm_upload_cohesion(mpm_handle* h, const double* c, unsigned n) {
         return MPM_OK;
     }
     if (n != h->n || h->prms.DP_tan_phi == 0) return MPM_ERR_ARG;
-    if (!h->p0) CK(h, dev_alloc(h, &h->p0, sizeof(double) * h->pitch));
-    if (is_mixed(h) && !h->p0f) CK(h, dev_alloc(h, &h->p0f, sizeof(float) * h->pitch));
+    // neither alone: a handle with one of them takes its contents for the cohesion
+    double* p0 = h->p0;
+    CK(h, dev_ensure(h, &p0, sizeof(double) * h->pitch));
+    if (is_mixed(h)) {
+        const cudaError_t e = dev_ensure(h, &h->p0f, sizeof(float) * h->pitch);
+        if (e != cudaSuccess && !h->p0) dev_free(h, p0);
+        CK(h, e);
+    }
+    h->p0 = p0;
     h->p2g_ready = false;
     if (n == 0) return MPM_OK;
     // cohesion to the device as given, then p0 = c / tan(phi) there (the same
@@ -1019,23 +1053,13 @@ int mpm_set_sort_interval(mpm_handle* h, int k) {
 namespace {
 
 int ensure_frame_scratch(mpm_handle* h) {
-    if (h->fr_f) return MPM_OK;
     const size_t p = h->pitch;
-    CK(h, dev_alloc(h, &h->fr_f, sizeof(float) * 7 * p));
-    CK(h, dev_alloc(h, &h->fr_status, p));
-    CK(h, dev_alloc(h, &h->fr_last, sizeof(int) * p));
-    CK(h, dev_alloc(h, &h->fr_i, sizeof(int) * 8 * (p + 1)));
-    CK(h, dev_alloc(h, &h->fr_rec, (sizeof(UpdPosRec) + sizeof(UpdJpRec) + sizeof(UpdStatusRec)) * p));
-    long long m = (long long)p + 1;
-    while (m > kScanTile) {
-        m = (m + kScanTile - 1) / kScanTile;
-        int* sums = nullptr;
-        int* scanned = nullptr;
-        CK(h, dev_alloc(h, &sums, sizeof(int) * m));
-        CK(h, dev_alloc(h, &scanned, sizeof(int) * m));
-        h->fr_scan_levels.push_back(sums);
-        h->fr_scan_levels.push_back(scanned);
-    }
+    CK(h, dev_ensure(h, &h->fr_f, sizeof(float) * 7 * p));
+    CK(h, dev_ensure(h, &h->fr_status, p));
+    CK(h, dev_ensure(h, &h->fr_last, sizeof(int) * p));
+    CK(h, dev_ensure(h, &h->fr_i, sizeof(int) * 8 * (p + 1)));
+    CK(h, dev_ensure(h, &h->fr_rec, (sizeof(UpdPosRec) + sizeof(UpdJpRec) + sizeof(UpdStatusRec)) * p));
+    CK(h, ensure_scan_levels(h, h->fr_scan_levels, (long long)p + 1, kScanTile));
     return MPM_OK;
 }
 
@@ -1161,13 +1185,7 @@ int mpm_step(mpm_handle* h, int nsteps, double* force_hist) {
     if (!h || nsteps < 0) return MPM_ERR_ARG;
     if (!h->uploaded) return MPM_ERR_STATE;
     if (nsteps == 0) return MPM_OK;
-    if (nsteps > h->force_steps_cap) {
-        CK(h, cudaStreamSynchronize(h->stream));
-        dev_free(h, h->force_steps);
-        h->force_steps = nullptr;
-        CK(h, dev_alloc(h, &h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
-        h->force_steps_cap = nsteps;
-    }
+    CK(h, dev_grow(h, &h->force_steps, &h->force_steps_cap, nsteps, sizeof(double) * 3));
     CK(h, cudaMemsetAsync(h->force_steps, 0, sizeof(double) * 3 * (size_t)nsteps, h->stream));
     SimParams3D& p = h->prms;
     if (is_mixed(h) && !h->p2g_ready) {
@@ -1874,13 +1892,7 @@ int mpm_multi_step(mpm_multi* m, int nsteps, double* force_hist) {
     SimParams3D& p = m->prms;
     for (mpm_handle* h : m->part) {
         CK(h, cudaSetDevice(h->device));
-        if (nsteps > h->force_steps_cap) {
-            CK(h, cudaStreamSynchronize(h->stream));
-            dev_free(h, h->force_steps);
-            h->force_steps = nullptr;
-            CK(h, dev_alloc(h, &h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
-            h->force_steps_cap = nsteps;
-        }
+        CK(h, dev_grow(h, &h->force_steps, &h->force_steps_cap, nsteps, sizeof(double) * 3));
         CK(h, cudaMemsetAsync(h->force_steps, 0, sizeof(double) * 3 * (size_t)nsteps, h->stream));
     }
     std::vector<double> total((size_t)3 * nsteps, 0.0);
@@ -2349,22 +2361,13 @@ int ensure_adjoint_buffers(mpm_handle* h, int nsteps, int every) {
         CK(h, dev_alloc(h, &b, sizeof(double) * 4 * gs));
         h->adj_gcache.push_back(b);
     }
-    h->ckpt_prms.resize(nck);
-    if (every > h->adj_rmc_cap) {
-        CK(h, cudaStreamSynchronize(h->stream));
-        dev_free(h, h->adj_rmc);
-        h->adj_rmc = nullptr;
-        h->adj_rmc_cap = 0;
-        CK(h, dev_alloc(h, &h->adj_rmc, sizeof(int) * (size_t)every));
-        h->adj_rmc_cap = every;
-    }
-    if (!h->adj_A) {
-        CK(h, dev_alloc(h, &h->adj_A, sizeof(double) * ADJ_ROWS * h->pitch));
-        CK(h, dev_alloc(h, &h->adj_cgrad, sizeof(double) * h->pitch));
-        CK(h, dev_alloc(h, &h->adj_Egrad, sizeof(double)));
-        CK(h, dev_alloc(h, &h->adj_gb7, sizeof(double) * 7 * (size_t)h->dp.gstride));
-        CK(h, dev_alloc(h, &h->adj_rmv, sizeof(double) * 10 * h->pitch));
-    }
+    if ((int)h->ckpt_prms.size() < nck) h->ckpt_prms.resize(nck);   // an earlier forward's stay until it is overwritten
+    CK(h, dev_grow(h, &h->adj_rmc, &h->adj_rmc_cap, every, sizeof(int)));
+    CK(h, dev_ensure(h, &h->adj_A, sizeof(double) * ADJ_ROWS * h->pitch));
+    CK(h, dev_ensure(h, &h->adj_cgrad, sizeof(double) * h->pitch));
+    CK(h, dev_ensure(h, &h->adj_Egrad, sizeof(double)));
+    CK(h, dev_ensure(h, &h->adj_gb7, sizeof(double) * 7 * gs));
+    CK(h, dev_ensure(h, &h->adj_rmv, sizeof(double) * 10 * h->pitch));
     // Last, since all but the first can be done without: the velocities of the
     // segment's substeps. With one buffer for all, the reverse sweep does the node
     // update of each substep again: 40 substeps of 20,000 points 3.14 -> 3.25 ms,
@@ -2446,13 +2449,7 @@ extern "C" int mpm_adjoint_forward(mpm_handle* h, int nsteps, int ckpt_every, do
     int r = ensure_adjoint_buffers(h, nsteps, ckpt_every);
     if (r) return r;
     if (is_mixed(h)) {
-        if (nsteps > h->adj_force_cap) {
-            CK(h, cudaStreamSynchronize(h->stream));
-            dev_free(h, h->adj_force);
-            h->adj_force = nullptr;
-            CK(h, dev_alloc(h, &h->adj_force, sizeof(double) * 3 * (size_t)nsteps));
-            h->adj_force_cap = nsteps;
-        }
+        CK(h, dev_grow(h, &h->adj_force, &h->adj_force_cap, nsteps, sizeof(double) * 3));
         h->adj_ready = false;
         if ((r = adjoint_forward_mixed(h, nsteps, ckpt_every))) return r;
         if (force_hist)
@@ -2464,14 +2461,9 @@ extern "C" int mpm_adjoint_forward(mpm_handle* h, int nsteps, int ckpt_every, do
         h->adj_ready = true;
         return MPM_OK;
     }
-    if (nsteps > h->force_steps_cap) {
-        CK(h, cudaStreamSynchronize(h->stream));
-        dev_free(h, h->force_steps);
-        h->force_steps = nullptr;
-        CK(h, dev_alloc(h, &h->force_steps, sizeof(double) * 3 * (size_t)nsteps));
-        h->force_steps_cap = nsteps;
-    }
+    CK(h, dev_grow(h, &h->force_steps, &h->force_steps_cap, nsteps, sizeof(double) * 3));
     if ((r = ensure_gvel64(h, nsteps))) return r;
+    h->adj_ready = false;   // the checkpoints of an earlier forward are overwritten from here on
     CK(h, cudaMemsetAsync(h->force_steps, 0, sizeof(double) * 3 * (size_t)nsteps, h->stream));
     for (int s = 0; s < nsteps; s++) {
         if (s % ckpt_every == 0) {
