@@ -32,6 +32,7 @@ ENTRY_POINTS = [
     ("mpm_params_parse_string", ctypes.c_int, [_pp, ctypes.c_char_p, ctypes.c_char_p, ctypes.c_int]),
     ("mpm_create", _hp, [_pp, ctypes.c_int, ctypes.c_uint, ctypes.c_int, _ip]),
     ("mpm_destroy", None, [_hp]),
+    ("mpm_release_memory", ctypes.c_int, [ctypes.c_int]),
     ("mpm_set_stream", ctypes.c_int, [_hp, ctypes.c_void_p]),
     ("mpm_update_constants", ctypes.c_int, [_hp, _pp]),
     ("mpm_upload_soa", ctypes.c_int, [_hp, _dp, ctypes.c_uint, ctypes.c_uint]),

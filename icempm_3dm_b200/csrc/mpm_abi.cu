@@ -166,8 +166,9 @@ int cuda_fail(mpm_handle* h, cudaError_t e, const char* what) {
 // 20,000-point gradient spent 44-52 ms, 7 of them on the device. The pool
 // keeps at most kPoolKeep bytes without an owner, returns the rest at the next
 // synchronisation, and all of it when the last handle goes while the device is
-// short of memory. Allocation and release are ordered on the handle's own
-// stream; the calls are safe from any thread.
+// short of memory, or when the program asks (mpm_release_memory). Allocation and
+// release are ordered on the handle's own stream; the calls are safe from any
+// thread.
 constexpr unsigned long long kPoolKeep = 1ull << 30;
 constexpr int kMaxDevices = 256;
 
@@ -1274,6 +1275,14 @@ int mpm_count(mpm_handle* h, unsigned* n) {
 }
 
 const char* mpm_last_error_string(void) { return g_last_error; }
+
+int mpm_release_memory(int device) {
+    if (device < 0 || device >= kMaxDevices) return MPM_ERR_ARG;
+    PoolTable& t = pools();
+    std::lock_guard<std::mutex> lock(t.mu);
+    if (t.pool[device]) CK(nullptr, cudaMemPoolTrimTo(t.pool[device], 0));
+    return MPM_OK;
+}
 
 int mpm_host_alloc(size_t bytes, void** ptr) {
     if (!ptr) return MPM_ERR_ARG;

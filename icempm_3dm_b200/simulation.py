@@ -265,6 +265,13 @@ class MPMHandle:
         return adj[:, :n]
 
 
+def release_memory(device=0):
+    """Returns the device memory that destroyed handles left with the library
+    for the next ones (at most 1 GiB) to the driver, for other users of the
+    device (mpm_release_memory)."""
+    check(LIB.mpm_release_memory(int(device)), "mpm_release_memory")
+
+
 def pinned_empty(shape, dtype=np.float64):
     """An uninitialised array over page-locked host memory (mpm_host_alloc,
     the memory HostSideSOA::Allocate takes, host_side_soa.cpp:70-86): copies

@@ -101,6 +101,11 @@ mpm_handle* mpm_create(const SimParams3D* prms, int precision, unsigned capacity
                        int device, int* status);
 /* GPU_Partition_3D::~GPU_Partition_3D (gpu_partition_3d.cu:27-50). */
 void mpm_destroy(mpm_handle* h);
+/* New: returns to the driver the device memory that destroyed handles (and
+ * buffers given up by living ones) left with the library for the next ones,
+ * 1 GiB at most, so that other users of the device can have it. MPM_OK also
+ * where there is none. */
+int  mpm_release_memory(int device);
 /* Issue all later work of h on `cuda_stream` (a cudaStream_t); NULL restores
  * the handle's own stream. */
 int  mpm_set_stream(mpm_handle* h, void* cuda_stream);

@@ -47,6 +47,11 @@ def test_create_without_device_fails_cleanly():
     assert not h and st.value == 103
 
 
+def test_release_memory_without_any():
+    assert LIB.mpm_release_memory(0) == 0
+    assert LIB.mpm_release_memory(-1) == LIB.mpm_release_memory(1 << 20) != 0
+
+
 C_PROGRAM = r"""
 #include <stdio.h>
 #include <string.h>

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from icempm_3dm_b200 import PRECISION_FP64_SVD64, MPMHandle
+from icempm_3dm_b200 import PRECISION_FP64_SVD64, MPMHandle, release_memory
 from tests.helpers import perturbed_block
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +65,20 @@ def test_what_stays_reserved_is_bounded():
         assert before - torch.cuda.mem_get_info()[0] > 2 * KEEP
     torch.cuda.synchronize()
     assert before - torch.cuda.mem_get_info()[0] <= KEEP + (64 << 20)
+
+
+def test_what_stays_reserved_can_be_given_back():
+    release_memory()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    prms, soa = perturbed_block(n=1200, seed=1)
+    with MPMHandle(prms, 12_000_000) as h:
+        h.upload(soa)
+        h.step(2)
+        release_memory()                      # what a living handle holds stays with it
+        assert np.isfinite(h.download()).all()
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] > KEEP // 2
+    release_memory()
+    # a page of the driver's own bookkeeping at most
+    assert before - torch.cuda.mem_get_info()[0] <= 64 << 20
