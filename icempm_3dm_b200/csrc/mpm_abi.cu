@@ -6,6 +6,7 @@
 // and GPU_Implementation6 (gpu_implementation6.cpp); the kernels are in the
 // kernels_*.cuh / sort.cuh headers.
 
+#include <chrono>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -176,6 +177,8 @@ struct PoolTable {
     std::mutex mu;
     cudaMemPool_t pool[kMaxDevices] = {};
     int handles[kMaxDevices] = {};
+    std::chrono::steady_clock::time_point asked[kMaxDevices] = {};   // when `scarce` was found
+    bool scarce[kMaxDevices] = {};
 };
 PoolTable& pools() {
     static PoolTable* t = new PoolTable();   // outlives every handle, also at process exit
@@ -296,12 +299,19 @@ void pool_enter(int device) {
     std::lock_guard<std::mutex> lock(t.mu);
     t.handles[device]++;
 }
+// The driver's answer to how much memory is free takes 0.07 ms, and up to 27 where
+// other programs use the machine's GPUs: it is good for a second.
 void pool_leave(int device) {
     PoolTable& t = pools();
     std::lock_guard<std::mutex> lock(t.mu);
     if (--t.handles[device] > 0 || !t.pool[device]) return;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b < total_b / 8) cudaMemPoolTrimTo(t.pool[device], 0);
+    const auto now = std::chrono::steady_clock::now();
+    if (now - t.asked[device] > std::chrono::seconds(1)) {
+        size_t free_b = 0, total_b = 0;
+        t.scarce[device] = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b < total_b / 8;
+        t.asked[device] = now;
+    }
+    if (t.scarce[device]) cudaMemPoolTrimTo(t.pool[device], 0);
 }
 
 DevParams make_dev_params(const SimParams3D& p) {
