@@ -83,9 +83,12 @@ __device__ __forceinline__ void p2g_alone(const DevParams& P, const P2GPoint& q,
         double w = 1.0, d[3];
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            const double u = q.fx[j] - (double)o[j];
-            w *= o[j] == 1 ? 0.75 - u * u : 0.5 * (1.5 - fabs(u)) * (1.5 - fabs(u));
-            d[j] = -u * P.h;
+            // the polynomials of quad_weights: f may lie outside [0.5, 1.5) here (a
+            // coordinate in (-0.5, 0.5) of a cell below the grid has base 0)
+            const double f = q.fx[j];
+            const double u = o[j] == 0 ? 1.5 - f : (o[j] == 1 ? f - 1.0 : f - 0.5);
+            w *= o[j] == 1 ? 0.75 - u * u : 0.5 * u * u;
+            d[j] = ((double)o[j] - f) * P.h;
         }
         const long long ni = node_index(P, x, y, z);
         atomicAdd(grid + ni, w * q.mass);

@@ -67,3 +67,32 @@ def test_p2g_merge(kind, n):
         for k in range(4):
             scale = np.abs(ref[k]).max()
             assert np.abs(got[k] - ref[k]).max() <= bound * scale + 1e-300, (precision, accum, k)
+
+
+def test_p2g_of_points_outside_the_grid():
+    """The part of a stencil that lies in the grid, for points that leave it on
+    one to three sides, among them coordinates between -0.5 and 0.5 cells: their
+    base is 0 and their weights are not in [0, 1]."""
+    prms, soa, _ = gen.small_block(n=1000, seed=9, halo=3)
+    h = prms.cellsize
+    at = [[lo, -0.9, -0.3, 0.2, 4.7, g - 1.7, g - 0.6, g + 0.4]
+          for lo, g in ((-3.8, prms.GridXTotal), (-1.4, prms.GridY), (-1.4, prms.GridZ))]
+    x = np.stack(np.meshgrid(*at, indexing="ij")).reshape(3, -1)
+    n = x.shape[1]
+    rng = np.random.default_rng(1)
+    soa = np.ascontiguousarray(np.repeat(soa[:, :1], n, axis=1))
+    soa[POSX:POSX + 3] = x * h
+    soa[VELX:VELX + 3] = rng.standard_normal((3, n))
+    soa[BP00:BP00 + 9] = 5 * rng.standard_normal((9, n))
+    for k in (n, 300, 1):
+        ref, err = po.p2g(prms, soa, k)
+        assert err != 0
+        with MPMHandle(prms, n, PRECISION_FP64) as hd:
+            hd.upload(np.ascontiguousarray(soa[:, :k]))
+            hd.reset_grid()
+            hd.p2g()
+            assert 70 <= hd.error() <= 75
+            got = hd.grid(0)
+        for c in range(4):
+            # the order of the sums, as above
+            assert np.abs(got[c] - ref[c]).max() <= 1e-12 * np.abs(ref[c]).max() + 1e-300
