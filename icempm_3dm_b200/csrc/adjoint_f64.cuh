@@ -10,19 +10,22 @@
 //         wall masks; f_n = sum_i f_i
 //   G2P   v' = sum_i w v_i, C' = 4/h^2 sum_i w v_i d_ip^T, x' = x + dt v',
 //         F_tr = (I + dt C') F, F' = RM(F_tr, Jp, p0, mu, kappa) if crushed
-// The reverse of one substep runs three kernels, after recomputing the grid
-// of substep n from S_n:
+// A segment's substeps are recomputed from its checkpoint, each out of place: the
+// states, the sums and velocities of the nodes and the lists of the points that
+// crushed stay until the segment is reversed. The reverse of one substep then runs
+// four kernels:
+//   k_adj_rm_vjp    crushed points: vector-Jacobian product of the return map
 //   k_adj_g2p_rev   particles: adjoint of G2P (including the weight
-//                   gradients and the return map), velocity adjoints
-//                   scattered to the nodes
+//                   gradients), velocity adjoints scattered to the nodes
 //   k_adj_node_rev  nodes: adjoint of the node update (masks, contact
 //                   projection, force, clamp, division by the mass)
 //   k_adj_p2g_rev   particles: adjoint of P2G as a gather over each
 //                   particle's 27 nodes (no atomics), including the
 //                   Kirchhoff stress
-// The return map's vector-Jacobian product uses the local Jacobian taken by
-// forward-mode dual numbers through the same FP64 SVD and projection code
-// (one direction per input), so it follows every branch the forward took.
+// The vector-Jacobian product takes the local Jacobian by forward-mode dual
+// numbers through the code of the return map itself, its polar form and, for the
+// deformations which that leaves, its FP64 SVD (one direction per input), so it
+// follows every branch the forward took.
 #pragma once
 
 #include <climits>
@@ -330,9 +333,11 @@ __global__ void __launch_bounds__(BLOCK) k_adj_rm_vjp(DevParams P, AdjParams Q, 
 // ten particles to a warp): a lane's nodes are one long chain of loads and
 // FP64 operations, and with few particles that chain is the kernel's time. Three
 // lanes repeat the particle's own arithmetic, which costs more once the chip is
-// full: reverse sweep over 40 substeps of 3,000 points 2.85 -> 2.47 ms, 20,000
-// 3.59 -> 3.15, 100,000 6.06 -> 6.94, 500,000 21.2 -> 28.5. Three up to 192
-// points per SM (28,416), about where the three-lane blocks fill it once.
+// full. Reverse sweep over 40 substeps with one lane and with three, ms: 3,000
+// points 2.80 and 2.45, 10,000 3.09 and 2.74, 20,000 3.55 and 3.12, 25,000 3.60
+// and 3.54, 28,400 3.76 and 3.76, 33,000 3.91 and 3.93, 45,000 4.30 and 4.48,
+// 70,000 4.94 and 5.59, 100,000 6.03 and 6.88. So three up to 192 points per SM
+// (28,416), where the two meet: 1.6 (G2P) and 1.2 (P2G) waves of their blocks.
 constexpr int kRevSplitPerSM = 192;
 struct RevLane {
     int i, part;        // particle, x-layer (lane 0 of a particle writes its results)

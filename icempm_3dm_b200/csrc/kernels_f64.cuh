@@ -302,8 +302,9 @@ __device__ __forceinline__ void update_node_f64(const DevParams& P, double* vel,
 enum { kVelInPlace = 0, kVelClear = 1, kVelRecord = 2, kVelOnly = 3 };
 constexpr int kUpdateF64NodesPerThread = 2;
 template <int BLOCK, int MODE>
-__global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* grid, double* vel, double ind_x, double ind_y,
-                                                      double* __restrict__ sensor, double* __restrict__ force3) {
+__global__ void __launch_bounds__(BLOCK) k_update_f64(DevParams P, double* grid, double* vel, double ind_x,
+                                                      double ind_y, double* __restrict__ sensor,
+                                                      double* __restrict__ force3) {
     chain_wait();
     constexpr int NPT = kUpdateF64NodesPerThread;
     const long long idx0 = (long long)P.node_lo + (long long)blockIdx.x * (BLOCK * NPT) + threadIdx.x;
@@ -499,9 +500,11 @@ __global__ void __launch_bounds__(kG2PBlock, kG2PF64Blocks) k_g2p_f64(
     __shared__ double fs[10 * kG2PBlock];
     const unsigned fdst = (unsigned)__cvta_generic_to_shared(fs + threadIdx.x);
 #pragma unroll
-    for (int q = 0; q < 10; q++)
+    for (int q = 0; q < 10; q++) {
+        const double* const from = pts + (q < 9 ? MPM_FE00 + q : MPM_IDX_JP_INV) * pitch + i;
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
-                     :: "r"(fdst + 8 * kG2PBlock * q), "l"(pts + (q < 9 ? MPM_FE00 + q : MPM_IDX_JP_INV) * pitch + i) : "memory");
+                     :: "r"(fdst + 8 * kG2PBlock * q), "l"(from) : "memory");
+    }
     double vel[3], C[3][3];
     g2p_gather(P, grid, pos, vel, C, err);
     asm volatile("cp.async.wait_all;" ::: "memory");

@@ -91,7 +91,8 @@ struct mpm_handle {
 
     // mixed precision (MPM_PRECISION_MIXED): 28 rows of 4-byte words
     // (X 0-2, v 3-5, E 6-14, C 15-23, Jp 24, status 25, P 26, Q 27); the FP64
-    // SoA `pts` is then the staging copy for upload, download and sort
+    // SoA `pts` is then the staging copy for upload and download (and the
+    // adjoint), and its first row holds the upper halves of the utility words
     void* mx = nullptr;
     float* p0f = nullptr;
     float4* gacc = nullptr;
@@ -229,7 +230,8 @@ cudaError_t dev_alloc(mpm_handle* h, T** ptr, size_t bytes, bool optional = fals
             e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
         }
     }
-    if (e == cudaErrorMemoryAllocation && !optional && release_optional(h)) {   // and without what the handle can do without
+    // and without what the handle can do without
+    if (e == cudaErrorMemoryAllocation && !optional && release_optional(h)) {
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(&p, bytes, pool, h->own_stream);
     }
@@ -402,7 +404,8 @@ bool params_valid(const SimParams3D* p) {
 inline unsigned blocks_for(long long n, int tpb) { return (unsigned)((n + tpb - 1) / tpb); }
 
 void free_all(mpm_handle* h) {
-    dev_free(h, h->pts); dev_free(h, h->p0); dev_free(h, h->ids); dev_free(h, h->grid); dev_free(h, h->gvel64); dev_free(h, h->sensor);
+    dev_free(h, h->pts); dev_free(h, h->p0); dev_free(h, h->ids);
+    dev_free(h, h->grid); dev_free(h, h->gvel64); dev_free(h, h->sensor);
     dev_free(h, h->force_steps); dev_free(h, h->force_phase); dev_free(h, h->err);
     dev_free(h, h->pts_alt); dev_free(h, h->mx_alt); dev_free(h, h->p0_alt); dev_free(h, h->ids_alt);
     dev_free(h, h->s_bucket); dev_free(h, h->s_count); dev_free(h, h->s_start); dev_free(h, h->s_perm);
@@ -421,7 +424,8 @@ void free_all(mpm_handle* h) {
     dev_free(h, h->adj_rmv); dev_free(h, h->adj_rmc);
     for (int* p : h->scan_levels) dev_free(h, p);
     h->scan_levels.clear();
-    dev_free(h, h->fr_f); dev_free(h, h->fr_status); dev_free(h, h->fr_last); dev_free(h, h->fr_i); dev_free(h, h->fr_rec);
+    dev_free(h, h->fr_f); dev_free(h, h->fr_status); dev_free(h, h->fr_last);
+    dev_free(h, h->fr_i); dev_free(h, h->fr_rec);
     for (int* p : h->fr_scan_levels) dev_free(h, p);
     h->fr_scan_levels.clear();
     if (h->own_stream) {
@@ -506,7 +510,8 @@ int launch_p2g(mpm_handle* h, const double* src = nullptr, double* acc = nullptr
         if (h->gacc_q)
             chain(k_p2g_mixed<AccQ>, blocks_for(n, 128), 128, 0, h->stream, h->dp, mixed_state(h), n, acc_q(h), h->err);
         else
-            chain(k_p2g_mixed<AccF4>, blocks_for(n, 128), 128, 0, h->stream, h->dp, mixed_state(h), n, AccF4{h->gacc}, h->err);
+            chain(k_p2g_mixed<AccF4>, blocks_for(n, 128), 128, 0, h->stream, h->dp, mixed_state(h), n,
+                  AccF4{h->gacc}, h->err);
         CK_LAUNCH(h, "p2g mixed");
         return MPM_OK;
     }
@@ -523,11 +528,11 @@ int launch_update(mpm_handle* h, double ind_x, double ind_y, double* force3, int
     if (is_mixed(h)) {
         const unsigned nbm = blocks_for((long long)h->dp.node_hi - h->dp.node_lo, 256 * kUpdateNodesPerThread);
         if (h->gacc_q)
-            chain(k_update_mixed<256, AccQ>, nbm, 256, 0, h->stream, h->dp, acc_q(h), h->gvel, ind_x, ind_y, h->sensor,
-                                                           force3);
+            chain(k_update_mixed<256, AccQ>, nbm, 256, 0, h->stream, h->dp, acc_q(h), h->gvel, ind_x, ind_y,
+                  h->sensor, force3);
         else
-            chain(k_update_mixed<256, AccF4>, nbm, 256, 0, h->stream, h->dp, AccF4{h->gacc}, h->gvel, ind_x, ind_y, h->sensor,
-                                                           force3);
+            chain(k_update_mixed<256, AccF4>, nbm, 256, 0, h->stream, h->dp, AccF4{h->gacc}, h->gvel, ind_x, ind_y,
+                  h->sensor, force3);
         CK_LAUNCH(h, "update mixed");
         return MPM_OK;
     }
@@ -552,12 +557,10 @@ int launch_return_map_mixed(mpm_handle* h, int do_p2g) {
     h->rm_parity ^= 1;
     if (h->gacc_q)
         chain(k_return_map_mixed<AccQ>, h->num_sms * 4, 128, 0, h->stream, h->dp, mixed_state(h), h->rm_list,
-                                                                  h->rm_counts + cur, h->rm_counts + (cur ^ 1),
-                                                                  acc_q(h), do_p2g, h->err);
+              h->rm_counts + cur, h->rm_counts + (cur ^ 1), acc_q(h), do_p2g, h->err);
     else
         chain(k_return_map_mixed<AccF4>, h->num_sms * 4, 128, 0, h->stream, h->dp, mixed_state(h), h->rm_list,
-                                                                  h->rm_counts + cur, h->rm_counts + (cur ^ 1),
-                                                                  AccF4{h->gacc}, do_p2g, h->err);
+              h->rm_counts + cur, h->rm_counts + (cur ^ 1), AccF4{h->gacc}, do_p2g, h->err);
     CK_LAUNCH(h, "return map mixed");
     return MPM_OK;
 }
@@ -573,11 +576,11 @@ int launch_g2p2g_mixed(mpm_handle* h, int do_p2g, int record_pq, int store_vc) {
     // the warps' velocity boxes: kVBoxNodes float4 of dynamic shared memory per warp
     const size_t vsm = sizeof(float4) * (kFusedBlock / 32) * kVBoxNodes;
     if (h->gacc_q)
-        chain(k_g2p2g_mixed<AccQ>, blocks_for(n, kFusedBlock), kFusedBlock, vsm, h->stream, h->dp, mixed_state(h), n, h->gvel, acc_q(h), do_p2g, record_pq, store_vc, h->err, h->rm_list,
-            rm_count);
+        chain(k_g2p2g_mixed<AccQ>, blocks_for(n, kFusedBlock), kFusedBlock, vsm, h->stream, h->dp, mixed_state(h), n,
+              h->gvel, acc_q(h), do_p2g, record_pq, store_vc, h->err, h->rm_list, rm_count);
     else
-        chain(k_g2p2g_mixed<AccF4>, blocks_for(n, kFusedBlock), kFusedBlock, vsm, h->stream, h->dp, mixed_state(h), n, h->gvel, AccF4{h->gacc}, do_p2g, record_pq, store_vc, h->err, h->rm_list,
-            rm_count);
+        chain(k_g2p2g_mixed<AccF4>, blocks_for(n, kFusedBlock), kFusedBlock, vsm, h->stream, h->dp, mixed_state(h), n,
+              h->gvel, AccF4{h->gacc}, do_p2g, record_pq, store_vc, h->err, h->rm_list, rm_count);
     CK_LAUNCH(h, "g2p2g mixed");
     return MPM_OK;
 }
@@ -2551,8 +2554,8 @@ extern "C" int mpm_adjoint_backward(mpm_handle* h, const double* dL_dforce, doub
             const unsigned nb = rev_blocks(n, 128, split ? 3 : 1);
             chain(split ? k_adj_g2p_rev<128, 3> : k_adj_g2p_rev<128, 1>, nb, 128, 0, h->stream, dp, q, S[m], S[m + 1],
                   h->pitch, n, vel, h->adj_rmv, h->adj_A, h->adj_gb7);
-            chain(k_adj_node_rev<256>, blocks_for(dp.nodes, 256), 256, 0, h->stream, dp, sums, h->adj_gb7, ix, iy, dl[0],
-                  dl[1], dl[2]);
+            chain(k_adj_node_rev<256>, blocks_for(dp.nodes, 256), 256, 0, h->stream, dp, sums, h->adj_gb7, ix, iy,
+                  dl[0], dl[1], dl[2]);
             chain(split ? k_adj_p2g_rev<128, 3> : k_adj_p2g_rev<128, 1>, nb, 128, 0, h->stream, dp, q, S[m], h->pitch,
                   n, h->adj_gb7, h->adj_A, h->adj_Egrad);
             CK_LAUNCH(h, "adjoint kernels");

@@ -21,7 +21,8 @@ def _source(name):
 
 def _functions(text):
     """(name, parameter list, body) of each device function or kernel."""
-    for m in re.finditer(r"(?:__global__|__device__)[^;{}]*?\b(\w+)\s*\(((?:[^()]|\([^()]*\))*)\)\s*(?:const\s*)?\{", text):
+    head = r"(?:__global__|__device__)[^;{}]*?\b(\w+)\s*\(((?:[^()]|\([^()]*\))*)\)\s*(?:const\s*)?\{"
+    for m in re.finditer(head, text):
         if m.group(1) == "__launch_bounds__":
             continue
         depth, k = 1, m.end()
