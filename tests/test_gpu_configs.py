@@ -101,7 +101,10 @@ def test_block2m_fp64_with_lognormal_cohesion_matches_oracle_over_2000_substeps(
     configuration's 2,000 substeps. As for block250k: tight agreement while
     the FP64 atomics' rounding has met no discrete switch (400 substeps), and
     at 2,000 a GPU-oracle distance within 5x the GPU's own run-to-run spread
-    (floor 1e-3 in force, 1e-6 m in position)."""
+    (floor 1e-3 in force, 1e-6 m in position). The spread is the largest
+    distance between any two of four runs: one pair in eight happens to meet
+    the switches alike and lies 1e-7 m apart, the others 1e-6 to 2.4e-6 m, the
+    oracle 3.9e-6 m from either."""
     prms, soa, coh = gen.make_block(gen.CONFIGS["block2m"])
     n = soa.shape[1]
     perm = po.sort_permutation(prms, soa, n)
@@ -123,7 +126,11 @@ def test_block2m_fp64_with_lognormal_cohesion_matches_oracle_over_2000_substeps(
         return np.concatenate(hist), outs
 
     g1, o1 = gpu_run()
-    g2, o2 = gpu_run()
+    runs = [(g1, [o[POSX:POSX + 3].copy() for o in o1])]
+    for _ in range(3):
+        g, o = gpu_run()
+        runs.append((g, [out[POSX:POSX + 3].copy() for out in o]))
+    pairs = [(a, b) for k, a in enumerate(runs) for b in runs[:k]]
     sim = po.OracleSim(prms, soa, n, p0=p0, svd_mode=0, nthreads=os.cpu_count() or 1)
     ref_hist, ref_out, done = [], [], 0
     for m in marks:
@@ -137,9 +144,9 @@ def test_block2m_fp64_with_lognormal_cohesion_matches_oracle_over_2000_substeps(
     lines = []
     for k, m in enumerate(marks):
         e = rel(g1[:m], ref_hist[:m])
-        e_run = rel(g1[:m], g2[:m])
+        e_run = max(rel(a[0][:m], b[0][:m]) for a, b in pairs)
         x = float(np.abs(o1[k][POSX:POSX + 3] - ref_out[k][POSX:POSX + 3]).max())
-        x_run = float(np.abs(o1[k][POSX:POSX + 3] - o2[k][POSX:POSX + 3]).max())
+        x_run = max(float(np.abs(a[1][k] - b[1][k]).max()) for a, b in pairs)
         f = rel(o1[k][FE00:FE00 + 9], ref_out[k][FE00:FE00 + 9])
         flips = int(np.sum(crushed(o1[k]) != crushed(ref_out[k])))
         lines.append(f"{m} substeps: force {e:.2e} (GPU run to run {e_run:.2e}), positions {x:.2e} m "
