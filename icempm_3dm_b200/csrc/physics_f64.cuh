@@ -122,8 +122,9 @@ __device__ __forceinline__ DPParams dp_params(const DevParams& P) {
 // rotations, each with a square root and a division in a serial chain, and
 // that chain is the kernel's time (the crushed points rarely fill the chip):
 // 0.7 % of 500,000 points crushed, mixed return map with its launch 16.4 ->
-// 12.5 us per substep; a 3,001-point block's substep 31 -> 27 us. Against the
-// 64-bit SVD form over the strains of tests/test_gpu_return_map.py: 1e-12.
+// 12.5 us per substep; a 3,001-point block's substep 31 -> 27 us. Error of F
+// against the map in 40 digits, strains of 1e-6 to 0.4, apex and yield: at most
+// 5e-16, the 64-bit SVD form's 1.8e-15.
 
 __device__ __forceinline__ double tval(double x) { return x; }
 
